@@ -541,6 +541,14 @@ gal_status gal_integrate_workspace_size(const gal_solver_config* cfg, int64_t n,
   return GAL_OK;
 }
 
+gal_status gal_integrate_workspace_size_saves(const gal_solver_config* cfg, int64_t n, int64_t total_saves,
+                                              size_t* bytes) {
+  if (total_saves < 0) return fail(GAL_ERR_INVALID_ARGUMENT, "bad workspace query");
+  const gal_status st = gal_integrate_workspace_size(cfg, n, bytes);
+  if (st == GAL_OK && cfg->method == 8) *bytes = align256(*bytes) + sizeof(double) * (size_t)total_saves;
+  return st;
+}
+
 gal_status gal_set_team(int32_t blocks) {
   if (blocks < 0 || blocks > 1024) return fail(GAL_ERR_INVALID_ARGUMENT, "team blocks must be in [0, 1024]");
   g_team_blocks.store(blocks, std::memory_order_relaxed);
@@ -625,6 +633,27 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   a.resume = nullptr;
   a.queue_len = nullptr;
   const LaunchShape shape = launch_shape(cfg->method, cfg->adaptive);
+  // Dopri8 saves as one parallel pass afterwards (put_deferred_save) when the
+  // workspace has an entry per save. Not for one warp per orbit, whose component
+  // sums a per-save thread would not repeat bit for bit, and not for saves in
+  // host memory, which would cross the bus three times.
+  if (cfg->method == 8 && total > 0 && workspace_bytes >= align256(need) + sizeof(double) * (size_t)total &&
+      (p->is_mw || !dopri8_warp_per_orbit(shape, n, p->n))) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, out) != cudaSuccess) {
+      cudaGetLastError();
+    } else if (attr.type == cudaMemoryTypeDevice) {
+      a.defer = reinterpret_cast<double*>(ws + align256(need));
+      const cudaError_t em = cudaMemsetAsync(a.defer, 0xff, sizeof(double) * (size_t)total, s);  // NaN: not deferred
+      if (em != cudaSuccess) return cuda_fail(em, "clearing the save scratch");
+    }
+  }
+  auto finish = [&](cudaError_t e, const char* what) -> gal_status {
+    if (e != cudaSuccess) return cuda_fail(e, what);
+    if (!a.defer) return GAL_OK;
+    e = launch_deferred_saves8(a, p->is_mw, p->mw, p->d_comps, p->n, s);
+    return e == cudaSuccess ? GAL_OK : cuda_fail(e, "deferred saves launch");
+  };
   auto launch = [&]() {
     return cfg->method == 8 ? launch_integrate_dopri8(a, p->is_mw, p->mw, p->d_comps, p->n, shape, s)
                             : launch_integrate_dopri5(a, p->is_mw, p->mw, p->d_comps, p->n, shape, s);
@@ -632,8 +661,7 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   if (!cfg->schedule) {
     cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return cuda_fail(e, "clearing the work queue");
-    e = launch();
-    return e == cudaSuccess ? GAL_OK : cuda_fail(e, "integrate kernel launch");
+    return finish(launch(), "integrate kernel launch");
   }
   // two phases: a fraction of every span (a tenth by default), then longest remaining work first
   const SchedLayout L = sched_layout(n);
@@ -704,10 +732,9 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
       if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap == cudaStreamCaptureStatusNone)
         cudaStreamSynchronize(ts);
     }
-    return e == cudaSuccess ? GAL_OK : cuda_fail(e, "integrate kernel launch (second pass, teams)");
+    return finish(e, "integrate kernel launch (second pass, teams)");
   }
-  e = launch();
-  return e == cudaSuccess ? GAL_OK : cuda_fail(e, "integrate kernel launch (second pass)");
+  return finish(launch(), "integrate kernel launch (second pass)");
 }
 
 int32_t gal_tableau(int32_t method, double* c, double* a, double* b, double* e) {

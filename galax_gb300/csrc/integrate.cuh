@@ -78,6 +78,7 @@ struct IntegrateArgs {
   int32_t phase;
   double split_frac;                     // <= 0: single pass
   OrbitResume* resume;                   // [n]
+  double* defer;                         // Dopri8: start time of each deferred save's step [out_stride], or NULL
   const unsigned long long* queue_len;   // phase 1: number of entries in order (device)
 };
 
@@ -236,6 +237,26 @@ __device__ __forceinline__ void write_save(const IntegrateArgs& a, const OrbitSt
 __device__ __forceinline__ double save_tau(const IntegrateArgs& a, const OrbitState& s, int64_t k) {
   const double ts = a.save_offsets ? a.save_ts[s.save_base + k] : a.save_ts[k];
   return s.dir * ts;
+}
+
+// Dopri8 saves are partial steps of their own from the start of the step they
+// fall into, 13 stages each, and nothing later depends on them. With a scratch
+// entry per save (a.defer) the integration therefore only leaves each one its
+// start: the state goes where the save will be, the start time into the
+// scratch, and k_deferred_saves takes all partial steps at once afterwards, in
+// parallel over saves instead of one after the other inside the orbit's chain
+// (58 us each for a lone thread). Measured, default tolerances: one orbit over
+// 2 Gyr with 256 saves 20.6 -> 14.0 ms; a mock stream of 1,000 releases, whose
+// progenitor has a save per release, 61.1 -> 31.5 ms.
+// A save at the end of the step is the step's own result (the same length,
+// hence the same arithmetic).
+__device__ __forceinline__ void put_deferred_save(const IntegrateArgs& a, const OrbitState& s, double tau_k,
+                                                  const double* y1) {
+  const int64_t idx = save_index(a, s, s.save_i);
+  const bool at_end = tau_k == s.tnext;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) a.out[j * a.out_stride + idx] = at_end ? y1[j] : s.y[j];
+  if (!at_end) a.defer[idx] = s.dir * s.tau;
 }
 
 __device__ __forceinline__ void finish_orbit(const IntegrateArgs& a, OrbitState& s, int32_t st) {
@@ -592,7 +613,12 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
             s.tau = tprev_new;
             s.tnext = tnext_new;
           } else {
-            if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+            if (a.defer != nullptr) {
+              while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+                put_deferred_save(a, s, save_tau(a, s, s.save_i), y1);
+                ++s.save_i;
+              }
+            } else if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
               // Dopri8 with saves inside this step: keep (tau, y) for the sub-steps
               s.pending = 1;
 #pragma unroll

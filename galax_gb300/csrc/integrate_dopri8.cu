@@ -9,6 +9,15 @@ cudaError_t launch_integrate_dopri8(const IntegrateArgs& a, bool mw, const MWPar
   return launch_integrate<Dopri8>(a, mw, p, comps, ncomp, shape, stream);
 }
 
+cudaError_t launch_deferred_saves8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                   cudaStream_t stream) {
+  return launch_deferred_saves<Dopri8>(a, mw, p, comps, ncomp, stream);
+}
+
+bool dopri8_warp_per_orbit(const LaunchShape& shape, int64_t n, int ncomp) {
+  return use_warp_per_orbit(shape, n, ncomp);
+}
+
 cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, unsigned long long* tqueue,
                                    long long tcap, int blocks, size_t smem, cudaStream_t stream) {
   cudaError_t e =

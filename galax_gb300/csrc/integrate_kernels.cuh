@@ -3,6 +3,7 @@
 #pragma once
 
 #include "launch.h"
+#include "vjp.cuh"
 
 namespace gal {
 
@@ -72,6 +73,67 @@ __global__ void __launch_bounds__(kMaxBlock) k_integrate_table(IntegrateArgs a, 
   } else {
     integrate_loop<TB>(a, TablePot{s_comps, ncomp});
   }
+}
+
+// The partial steps that the integration deferred (put_deferred_save): one
+// thread per save, all independent. Entries of a.defer without a start time
+// (NaN) are saves that were written in place. The arithmetic is the inline
+// sub-step's, so saves are the same bits either way. For a static field
+// (dir tau_k - tau) dir = ts - t, t = dir tau: exact, the sign is +-1.
+template <class TB, class Pot>
+__device__ __forceinline__ void deferred_saves(const IntegrateArgs& a, const Pot& pot) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.out_stride;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double t = a.defer[i];
+    if (isnan(t)) continue;
+    const double hs = (a.save_offsets ? a.save_ts[i] : a.save_ts[i / a.n]) - t;
+    double y[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) y[j] = a.out[j * a.out_stride + i];
+    rk_step_plain<TB>(pot, y, hs, t);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) a.out[j * a.out_stride + i] = y[j];
+  }
+}
+
+template <class TB>
+__global__ void __launch_bounds__(128) k_deferred_saves_mw(IntegrateArgs a, MWParams p) {
+  deferred_saves<TB>(a, MWPot{p});
+}
+
+template <class TB, bool TIMED>
+__global__ void __launch_bounds__(128) k_deferred_saves_table(IntegrateArgs a, const DevComp* comps, int ncomp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  DevComp* s_comps = reinterpret_cast<DevComp*>(smem_raw);
+  for (int i = threadIdx.x; i < ncomp; i += blockDim.x) s_comps[i] = comps[i];
+  __syncthreads();
+  if constexpr (TIMED) {
+    deferred_saves<TB>(a, TimedTablePot{s_comps, ncomp, a.lin});
+  } else {
+    deferred_saves<TB>(a, TablePot{s_comps, ncomp});
+  }
+}
+
+// One warp per block while that gives every SM sub-partition at most one warp.
+template <class TB>
+cudaError_t launch_deferred_saves(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                  cudaStream_t stream) {
+  const int block = a.out_stride > 128LL * device_sm_count() ? 128 : 32;
+  const int64_t cap = 64LL * device_sm_count();
+  int64_t grid = (a.out_stride + block - 1) / block;
+  if (grid > cap) grid = cap;
+  if (mw) {
+    k_deferred_saves_mw<TB><<<(unsigned)grid, block, 0, stream>>>(a, p);
+    return cudaGetLastError();
+  }
+  const size_t smem = sizeof(DevComp) * (size_t)ncomp;
+  auto kernel = a.lin ? k_deferred_saves_table<TB, true> : k_deferred_saves_table<TB, false>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  kernel<<<(unsigned)grid, block, smem, stream>>>(a, comps, ncomp);
+  return cudaGetLastError();
 }
 
 // One warp per orbit (composites with many components): the lanes split the

@@ -344,7 +344,17 @@ __global__ void __launch_bounds__(128, 1) k_integrate_mw_team(IntegrateArgs a, M
           s.tau = tprev_new;
           s.tnext = tnext_new;
         } else {
-          if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+          if (a.defer != nullptr) {
+            while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+              const bool at_end = save_tau(a, s, s.save_i) == s.tnext;  // as put_deferred_save
+              if (owner) {
+                team_write_save(a, s, s.save_i, j0, at_end ? y1o0 : yo0);
+                team_write_save(a, s, s.save_i, j1, at_end ? y1o1 : yo1);
+              }
+              if (warp == 3 && !at_end) a.defer[save_index(a, s, s.save_i)] = s.dir * s.tau;
+              ++s.save_i;
+            }
+          } else if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
             // saves inside this step: keep (tau, y) for the sub-steps
             s.pending = 1;
 #pragma unroll

@@ -37,6 +37,11 @@ cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, un
                                    long long tcap, int blocks, size_t smem, cudaStream_t stream);
 cudaError_t launch_integrate_dopri8_exclusive(const IntegrateArgs& a, const MWParams& p, int variant, int block,
                                               int grid, size_t smem, cudaStream_t stream);
+// Dopri8 saves left to a.defer (put_deferred_save), after the integration on the same stream.
+cudaError_t launch_deferred_saves8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                   cudaStream_t stream);
+// Whether such a batch runs one warp per orbit, whose sums have another order than one thread's.
+bool dopri8_warp_per_orbit(const LaunchShape& shape, int64_t n, int ncomp);
 constexpr size_t kExclusiveSmem = 120 * 1024;
 
 int device_sm_count();

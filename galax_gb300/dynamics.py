@@ -30,6 +30,12 @@ from .potential import KMS_TO_KPC_MYR, AbstractPotential
 UNBOUNDED_MAX_STEPS = 2**20
 
 
+# Dopri8's scratch for saves (8 bytes each): kept with the workspace up to the first
+# bound (64 MB), allocated per call up to the second (4 GB), not used beyond.
+SAVE_SCRATCH_KEPT = 2**23
+SAVE_SCRATCH_MAX = 2**29
+
+
 def _torch():
     import torch
 
@@ -316,8 +322,17 @@ def integrate(
         ordp = ordt.data_ptr()
     L = _lib.load()
     nbytes = C.c_size_t()
-    _lib.check(L.gal_integrate_workspace_size(C.byref(cfg), n, C.byref(nbytes)), "gal_integrate_workspace_size")
-    ws = (workspace or _WS).get(nbytes.value)
+    total = shape[1] if save_offsets is not None else shape[1] * n
+    # a large save scratch (Dopri8, 8 bytes per save) is this call's alone instead of staying with the workspace
+    own = total > SAVE_SCRATCH_KEPT
+    if total > SAVE_SCRATCH_MAX:
+        total = 0
+    _lib.check(L.gal_integrate_workspace_size_saves(C.byref(cfg), n, total, C.byref(nbytes)),
+               "gal_integrate_workspace_size_saves")
+    if own and cfg.method == 8:
+        ws = torch.empty(nbytes.value, dtype=torch.uint8, device="cuda")
+    else:
+        ws = (workspace or _WS).get(nbytes.value)
     st = torch.cuda.current_stream().cuda_stream
     _lib.check(
         L.gal_integrate(

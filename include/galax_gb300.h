@@ -163,6 +163,13 @@ typedef struct gal_solver_config {
  * cfg->schedule = 1 a 128-byte resume record per orbit plus ordering arrays). */
 GAL_API gal_status gal_integrate_workspace_size(const gal_solver_config* cfg, int64_t n, size_t* bytes);
 
+/* The same, plus room for Dopri8's save scratch (8 bytes per save, total_saves
+ * over all orbits). With a workspace of this size gal_integrate takes the
+ * partial steps to save times as one parallel pass after the integration
+ * instead of inside it; the results are bitwise the same. */
+GAL_API gal_status gal_integrate_workspace_size_saves(const gal_solver_config* cfg, int64_t n, int64_t total_saves,
+                                              size_t* bytes);
+
 /* Integrate n orbits from t0[i] to t1[i] (t1 < t0 integrates backwards) and
  * write the state at each orbit's save times. Replaces diffrax.diffeqsolve with
  * SaveAt(ts=...) as driven by galax's Integrator / OrbitSolver
@@ -180,7 +187,8 @@ GAL_API gal_status gal_integrate_workspace_size(const gal_solver_config* cfg, in
  * status    : [n] gal_orbit_status (may be NULL)
  * steps     : [n] accepted steps per orbit (may be NULL)
  * order     : optional [n] permutation: the work queue hands orbits out in this order
- * workspace : device scratch of at least gal_integrate_workspace_size bytes */
+ * workspace : device scratch of at least gal_integrate_workspace_size bytes
+ *             (gal_integrate_workspace_size_saves bytes for Dopri8's fast saves) */
 GAL_API gal_status gal_integrate(const gal_potential* pot, const gal_solver_config* cfg, const double* y0, const double* t0,
                          const double* t1, const int64_t* save_offsets, const double* save_ts, int64_t n_saves,
                          double* out, int32_t* status, int64_t* steps, const int32_t* order, int64_t n,
