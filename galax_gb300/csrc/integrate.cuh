@@ -36,7 +36,7 @@ namespace gal {
 
 enum { ORBIT_OK = 0, ORBIT_MAX_STEPS = 1, ORBIT_DT_MIN = 2, ORBIT_NONFINITE = 3 };
 
-constexpr int kTeamLanes = 32;  // orbits per four-warp team block (integrate_team.cuh)
+constexpr int kTeamLanes = 16;  // orbits per four-warp team block (integrate_team.cuh)
 
 // Everything needed to continue an orbit exactly where a first pass parked it
 // (state, step times, controller memory, counters, save cursor). 128 bytes.
@@ -269,31 +269,104 @@ __device__ __forceinline__ void finish_orbit(const IntegrateArgs& a, OrbitState&
   s.orbit = -1;
 }
 
+// Hairer, Norsett & Wanner (1993) II.4, as used by diffrax when dt0 is None: in
+// two parts, around the field evaluation at Y = y + h0 dir F0 (team blocks
+// evaluate it together).
+struct InitialStep {
+  double sc[6], h0, d1;
+};
+
+__device__ __forceinline__ InitialStep initial_probe(const IntegrateArgs& a, const double* y, const double* F0) {
+  InitialStep s;
+  double q[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) s.sc[j] = fma(fabs(y[j]), a.rtol, a.atol);
+#pragma unroll
+  for (int j = 0; j < 6; ++j) q[j] = y[j] / s.sc[j];
+  const double d0 = rms6(q);
+#pragma unroll
+  for (int j = 0; j < 6; ++j) q[j] = F0[j] / s.sc[j];
+  s.d1 = rms6(q);
+  const bool cond = (d0 < 1e-5) || (s.d1 < 1e-5);
+  s.h0 = cond ? 1e-6 : 0.01 * (d0 / s.d1);
+  return s;
+}
+
+template <class TB>
+__device__ __forceinline__ double initial_finish(const InitialStep& s, const double* F0, const double* F1) {
+  double q[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) q[j] = (F1[j] - F0[j]) / s.sc[j];
+  const double d2 = rms6(q) / s.h0;
+  const double maxd = fmax(s.d1, d2);
+  const double h1 = (maxd <= 1e-15) ? fmax(1e-6, s.h0 * 1e-3) : pow(0.01 / maxd, 1.0 / (TB::ORDER + 1.0));
+  return fmin(100.0 * s.h0, h1);
+}
+
 template <class TB, class Pot>
 __device__ __forceinline__ double initial_step(const IntegrateArgs& a, const Pot& pot, const double* y,
                                                const double* F0, double dir, double t) {
-  // Hairer, Norsett & Wanner (1993) II.4, as used by diffrax when dt0 is None.
-  double sc[6], q[6];
-#pragma unroll
-  for (int j = 0; j < 6; ++j) sc[j] = fma(fabs(y[j]), a.rtol, a.atol);
-#pragma unroll
-  for (int j = 0; j < 6; ++j) q[j] = y[j] / sc[j];
-  const double d0 = rms6(q);
-#pragma unroll
-  for (int j = 0; j < 6; ++j) q[j] = F0[j] / sc[j];
-  const double d1 = rms6(q);
-  const bool cond = (d0 < 1e-5) || (d1 < 1e-5);
-  const double h0 = cond ? 1e-6 : 0.01 * (d0 / d1);
+  const InitialStep s = initial_probe(a, y, F0);
   double Y[6], F1[6];
 #pragma unroll
-  for (int j = 0; j < 6; ++j) Y[j] = fma(h0 * dir, F0[j], y[j]);
-  field(pot, Y, F1, fma(h0, dir, t));
+  for (int j = 0; j < 6; ++j) Y[j] = fma(s.h0 * dir, F0[j], y[j]);
+  field(pot, Y, F1, fma(s.h0, dir, t));
+  return initial_finish<TB>(s, F0, F1);
+}
+
+// Spans, save cursor and initial state of orbit s.orbit.
+__device__ __forceinline__ void begin_orbit(const IntegrateArgs& a, OrbitState& s, double t0, double t1) {
+  const int64_t o = s.orbit;
+  if (a.save_offsets) {
+    s.save_base = a.save_offsets[o];
+    s.save_end = a.save_offsets[o + 1] - s.save_base;
+  } else {
+    s.save_base = o;
+    s.save_end = a.n_saves;
+  }
+  s.pending = 0;
+  s.dir = (t0 < t1) ? 1.0 : -1.0;
+  s.tau0 = s.dir * t0;
+  s.tau1 = s.dir * t1;
+  if (a.phase == 1) return;
 #pragma unroll
-  for (int j = 0; j < 6; ++j) q[j] = (F1[j] - F0[j]) / sc[j];
-  const double d2 = rms6(q) / h0;
-  const double maxd = fmax(d1, d2);
-  const double h1 = (maxd <= 1e-15) ? fmax(1e-6, h0 * 1e-3) : pow(0.01 / maxd, 1.0 / (TB::ORDER + 1.0));
-  return fmin(100.0 * h0, h1);
+  for (int j = 0; j < 6; ++j) s.y[j] = a.y0[j * a.n + o];
+  s.save_i = 0;
+  s.nsteps = 0;
+  s.naccepted = 0;
+  s.tau = s.tau0;
+  s.prev_inv = 1.0;
+  s.prev_prev_inv = 1.0;
+  s.at_dtmin = 0;
+  s.status = ORBIT_OK;
+}
+
+// Phase 1: continue a parked orbit exactly.
+__device__ __forceinline__ void resume_orbit(const IntegrateArgs& a, OrbitState& s) {
+  const OrbitResume& r = a.resume[s.orbit];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) s.y[j] = r.y[j];
+  s.tau = r.tau;
+  s.tnext = r.tnext;
+  s.prev_inv = r.prev_inv;
+  s.prev_prev_inv = r.prev_prev_inv;
+  s.nsteps = r.nsteps;
+  s.naccepted = r.naccepted;
+  s.save_i = r.save_i;
+  s.at_dtmin = r.at_dtmin;
+  s.status = r.status;
+}
+
+// First step's end from its length dt (a.dt0 or initial_step's).
+__device__ __forceinline__ void first_step(const IntegrateArgs& a, OrbitState& s, double dt) {
+  if (a.adaptive) {
+    if (a.dtmax > 0.0) dt = fmin(dt, a.dtmax);
+    if (a.dtmin > 0.0) {
+      s.at_dtmin = dt <= a.dtmin;
+      dt = fmax(dt, a.dtmin);
+    }
+  }
+  s.tnext = fmin(s.tau + dt, s.tau1);
 }
 
 // Queue position of a thread's first orbit. The queue is ordered longest work
@@ -342,43 +415,12 @@ __device__ __forceinline__ bool start_orbit(const IntegrateArgs& a, const Pot& p
     const int64_t o = a.order ? (int64_t)a.order[k] : (int64_t)k;
     s.orbit = o;
     const double t0 = a.t0[o], t1 = a.t1[o];
-    if (a.save_offsets) {
-      s.save_base = a.save_offsets[o];
-      s.save_end = a.save_offsets[o + 1] - s.save_base;
-    } else {
-      s.save_base = o;
-      s.save_end = a.n_saves;
-    }
-    s.pending = 0;
-    s.dir = (t0 < t1) ? 1.0 : -1.0;
-    s.tau0 = s.dir * t0;
-    s.tau1 = s.dir * t1;
-    if (a.phase == 1) {  // continue a parked orbit exactly
-      const OrbitResume& r = a.resume[o];
-#pragma unroll
-      for (int j = 0; j < 6; ++j) s.y[j] = r.y[j];
-      s.tau = r.tau;
-      s.tnext = r.tnext;
-      s.prev_inv = r.prev_inv;
-      s.prev_prev_inv = r.prev_prev_inv;
-      s.nsteps = r.nsteps;
-      s.naccepted = r.naccepted;
-      s.save_i = r.save_i;
-      s.at_dtmin = r.at_dtmin;
-      s.status = r.status;
+    begin_orbit(a, s, t0, t1);
+    if (a.phase == 1) {
+      resume_orbit(a, s);
       field(pot, s.y, s.F0, s.dir * s.tau);
       return true;
     }
-#pragma unroll
-    for (int j = 0; j < 6; ++j) s.y[j] = a.y0[j * a.n + o];
-    s.save_i = 0;
-    s.nsteps = 0;
-    s.naccepted = 0;
-    s.tau = s.tau0;
-    s.prev_inv = 1.0;
-    s.prev_prev_inv = 1.0;
-    s.at_dtmin = 0;
-    s.status = ORBIT_OK;
     if (t0 == t1) {  // nothing to integrate: every save is the initial state
       for (; s.save_i < s.save_end; ++s.save_i) write_save(a, s, s.save_i, s.y);
       finish_orbit(a, s, ORBIT_OK);
@@ -389,18 +431,9 @@ __device__ __forceinline__ bool start_orbit(const IntegrateArgs& a, const Pot& p
       continue;
     }
     field(pot, s.y, s.F0, t0);
-    double dt;
-    if (a.adaptive) {
-      dt = a.dt0 > 0.0 ? a.dt0 : initial_step<TB>(a, pot, s.y, s.F0, s.dir, t0);
-      if (a.dtmax > 0.0) dt = fmin(dt, a.dtmax);
-      if (a.dtmin > 0.0) {
-        s.at_dtmin = dt <= a.dtmin;
-        dt = fmax(dt, a.dtmin);
-      }
-    } else {
-      dt = a.dt0;
-    }
-    s.tnext = fmin(s.tau + dt, s.tau1);
+    double dt = a.dt0;
+    if (a.adaptive && !(a.dt0 > 0.0)) dt = initial_step<TB>(a, pot, s.y, s.F0, s.dir, t0);
+    first_step(a, s, dt);
     return true;
   }
 }

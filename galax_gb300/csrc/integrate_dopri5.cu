@@ -9,12 +9,14 @@ cudaError_t launch_integrate_dopri5(const IntegrateArgs& a, bool mw, const MWPar
   return launch_integrate<Dopri5>(a, mw, p, comps, ncomp, shape, stream);
 }
 
-cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, unsigned long long* tqueue,
-                                  long long tcap, int blocks, size_t smem, cudaStream_t stream) {
-  cudaError_t e =
-      cudaFuncSetAttribute(k_integrate_mw_team<Dopri5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_integrate_mw_team<Dopri5><<<(unsigned)blocks, 128, smem, stream>>>(a, p, tqueue, tcap);
+cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, long long base, int blocks, size_t smem,
+                                  cudaStream_t stream) {
+  if (smem > 0) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_integrate_mw_team<Dopri5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_integrate_mw_team<Dopri5><<<(unsigned)blocks, 128, smem, stream>>>(a, p, base);
   return cudaGetLastError();
 }
 

@@ -18,12 +18,14 @@ bool dopri8_warp_per_orbit(const LaunchShape& shape, int64_t n, int ncomp) {
   return use_warp_per_orbit(shape, n, ncomp);
 }
 
-cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, unsigned long long* tqueue,
-                                   long long tcap, int blocks, size_t smem, cudaStream_t stream) {
-  cudaError_t e =
-      cudaFuncSetAttribute(k_integrate_mw_team<Dopri8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_integrate_mw_team<Dopri8><<<(unsigned)blocks, 128, smem, stream>>>(a, p, tqueue, tcap);
+cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, long long base, int blocks, size_t smem,
+                                  cudaStream_t stream) {
+  if (smem > 0) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_integrate_mw_team<Dopri8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_integrate_mw_team<Dopri8><<<(unsigned)blocks, 128, smem, stream>>>(a, p, base);
   return cudaGetLastError();
 }
 

@@ -1,29 +1,41 @@
-// Four-warp teams for the longest orbits of an adaptive Dopri5 or Dopri8
-// batch in the Milky Way model.
+// Four-warp teams with paired stages: the latency-optimal arrangement for few
+// or long orbits in the Milky Way model.
 //
-// The orbits that run longest set the duration of an uneven batch, and a lone
-// orbit is latency-bound: a GB300 FP64 warp instruction holds its
-// sub-partition's FP64 pipe for ~64 cycles however few lanes are active. A
-// team block (4 warps, one per sub-partition) integrates 32 orbits, one per
-// lane, and splits every field evaluation over the four warps:
-//   warp 0: the spheres' radius and the shared reciprocal (mw_ir, mw_recip);
+// A lone orbit is bound by its chain of FP64 instructions: a GB300 FP64 warp
+// instruction holds its sub-partition's FP64 pipe for 64 cycles (76 with all
+// four pipes busy) however few lanes are active. A team block (4 warps, one per
+// sub-partition) integrates 16 orbits and shortens the chain twice.
+//
+// Two stages per round. The force depends on the position alone, so with
+// F_i = (V_i, -g(X_i)), V_i = v + hs sum_{l<i} a_il (-g_l) and
+// X_i = x + hs sum_{l<i} a_il V_l, the position X_{i+1} needs the velocity V_i
+// and with it only the gradients up to g_{i-1}: gradients i and i + 1 do not
+// depend on one another. The stages are taken in pairs (1,2), (3,4), ...: lanes
+// 0-15 hold stage i of the block's 16 orbits and lanes 16-31 stage i + 1, and
+// one pass of the gradient code serves both. Dopri5 takes 3 rounds a step
+// instead of 6, Dopri8 6 (and one for the next step's first slope) instead of 13.
+//
+// Four warps per gradient:
+//   warp 0: the spheres' radius, the shared reciprocal, the bulge and nucleus;
 //   warp 1: the radius and the NFW halo's log(1 + r / r_s) (mw_halo_log);
+//   warp 2: the radius and the halo's factor;
 //   warp 3: the Miyamoto-Nagai disk (mw_disk);
-// and warps 0-2 own state components (w, w + 3), form the stage states and
-// combine the pieces (mw_f) into their gradient component. Step control is
-// computed redundantly by all four warps from the same shared-memory values.
-// Every operation matches the one-thread-per-orbit kernel (k_integrate_mw with
+// warps 0-2 own state components (w, w + 3), form their stage states and
+// combine the pieces into their gradient component. Step control is computed
+// redundantly by all four warps from the same shared-memory values. Every
+// operation matches the one-thread-per-orbit kernel (k_integrate_mw with
 // MWPot::grad, integrate_loop), so results are bitwise identical.
 //
-// Dopri5 is FSAL: a step's last stage is the next step's first slope. Dopri8
-// is not, and follows integrate_loop's non-FSAL branch: after an accepted step
-// the slope at the new state is one more team round, and saves inside an
-// accepted step are written by sub-steps of the partial length from the
-// step's start (the orbit stays "pending" until its last save of the step),
-// each one RK evaluation of its own.
+// Measured (constant step, one block per SM): a Dopri8 step 17.3 us, where the
+// one-thread kernel takes 58 us and a team of 32 orbits with one stage per round
+// took about 36; a Dopri5 step 9.2 us instead of 26.
 //
-// Used for the second pass of the two-pass schedule only: every orbit resumes
-// from its parked state.
+// Dopri5 is FSAL: a step's last stage is the next step's first slope, and its
+// state is the solution. Dopri8 is not: after an accepted step the slope at the
+// new state is one more round, and without a save scratch (a.defer) the saves
+// inside an accepted step are written by sub-steps of the partial length (the
+// orbit stays "pending" until its last save of the step), each one RK
+// evaluation of its own.
 #pragma once
 
 #include "integrate.cuh"
@@ -31,28 +43,36 @@
 namespace gal {
 
 struct TeamShared {
-  // field-evaluation exchange, double-buffered by round parity
-  double pos[2][3][kTeamLanes];
-  double u[2][kTeamLanes], us[2][kTeamLanes], izb[2][kTeamLanes];
-  double ir[2][kTeamLanes], L[2][kTeamLanes];
-  double inv_dh[2][kTeamLanes], inv_db2[2][kTeamLanes], inv_dn2[2][kTeamLanes];
+  // field-evaluation exchange: lane = 16 * (stage of the pair) + orbit
+  double pos[3][32];
+  double u[32], us[32], izb[32];
+  double A[32], B[32], inv_dh[32], ir[32], L[32];
   // controller exchange
   double y1[6][kTeamLanes], err[6][kTeamLanes];
   long long slot[kTeamLanes];
 };
 
-// Y_j = y_j + hs sum_{l<I} A[I][l] F_l,j for one component (stage_state's arithmetic).
-template <class TB, int I>
-__device__ __forceinline__ double stage_comp(double yj, double hs, const double (&Fj)[TB::S]) {
-  double acc = 0.0;
-  bool first = true;
-  static_for<0, I>([&](auto l) {
+// One coefficient of each half of the lanes; zero coefficients add nothing, as
+// in stage_state, where their terms do not exist.
+template <bool FIRST>
+__device__ __forceinline__ double pair_term(bool hi, double ca, double cb, double F, double acc) {
+  const double c = hi ? cb : ca;
+  if constexpr (FIRST) return c * F;
+  const double t = fma(c, F, acc);
+  if (ca != 0.0 && cb != 0.0) return t;
+  return (hi ? cb : ca) != 0.0 ? t : acc;
+}
+
+// Y_j = y_j + hs sum_{l<I} A[I][l] F_l,j for one component (stage_state's
+// arithmetic): row IA on lanes 0-15, row IB on lanes 16-31.
+template <class TB, int IA, int IB>
+__device__ __forceinline__ double pair_row(bool hi, double yj, double hs, const double (&Fj)[TB::S]) {
+  static_assert(TB::A[IA][0] != 0.0 && TB::A[IB][0] != 0.0, "rows start with their first slope");
+  double acc = pair_term<true>(hi, TB::A[IA][0], TB::A[IB][0], Fj[0], 0.0);
+  static_for<1, (IA > IB ? IA : IB)>([&](auto l) {
     constexpr int L = decltype(l)::value;
-    constexpr double c = TB::A[I][L];
-    if constexpr (c != 0.0) {
-      acc = first ? c * Fj[L] : fma(c, Fj[L], acc);
-      first = false;
-    }
+    constexpr double ca = L < IA ? TB::A[IA][L] : 0.0, cb = L < IB ? TB::A[IB][L] : 0.0;
+    if constexpr (ca != 0.0 || cb != 0.0) acc = pair_term<false>(hi, ca, cb, Fj[L], acc);
   });
   return fma(hs, acc, yj);
 }
@@ -101,37 +121,36 @@ __device__ __forceinline__ double dense_comp(double y0j, double hs, const double
   return fma(hs, acc, y0j);
 }
 
-// One team field evaluation: the owners (warps 0-2) have put the position
-// components in pos[b][w]; returns warp w's gradient component (w < 3).
-__device__ __forceinline__ double team_grad(TeamShared& sh, int b, int warp, int lane, const MWParams& p) {
+// One round of field evaluations, a point per lane: the owners (warps 0-2) hold
+// their position component `q`; returns warp w's gradient component (w < 3).
+__device__ __forceinline__ double team_grad(TeamShared& sh, int warp, int lane, const MWParams& p, double q) {
+  if (warp < 3) sh.pos[warp][lane] = q;
   __syncthreads();  // positions written
-  const double x = sh.pos[b][0][lane], y = sh.pos[b][1][lane], z = sh.pos[b][2][lane];
-  if (warp == 0) {
+  const double x = sh.pos[0][lane], y = sh.pos[1][lane], z = sh.pos[2][lane];
+  if (warp == 3) {
+    const MWDisk d = mw_disk(p, x, y, z);
+    sh.u[lane] = d.u;
+    sh.us[lane] = d.us;
+    sh.izb[lane] = d.izb;
+  } else {  // mw_f's products where their factors are
     double r;
     const double ir = mw_ir(x, y, z, r);
-    const MWRecip c = mw_recip(p, r);
-    sh.ir[b][lane] = ir;
-    sh.inv_dh[b][lane] = c.inv_dh;
-    sh.inv_db2[b][lane] = c.inv_db2;
-    sh.inv_dn2[b][lane] = c.inv_dn2;
-  } else if (warp == 1) {
-    double r;
-    mw_ir(x, y, z, r);
-    sh.L[b][lane] = mw_halo_log(p, r);
-  } else if (warp == 3) {
-    const MWDisk d = mw_disk(p, x, y, z);
-    sh.u[b][lane] = d.u;
-    sh.us[b][lane] = d.us;
-    sh.izb[b][lane] = d.izb;
+    if (warp == 0) {
+      const MWRecip c = mw_recip(p, r);
+      sh.B[lane] = ir * fma(p.Gm_b, c.inv_db2, p.Gm_n * c.inv_dn2);
+      sh.inv_dh[lane] = c.inv_dh;
+    } else if (warp == 1) {
+      sh.L[lane] = mw_halo_log(p, r);
+    } else {
+      sh.A[lane] = p.Gm_h * (ir * ir);
+      sh.ir[lane] = ir;
+    }
   }
   __syncthreads();  // pieces written
   if (warp > 2) return 0.0;
-  const MWRecip c{sh.inv_dh[b][lane], sh.inv_db2[b][lane], sh.inv_dn2[b][lane]};
-  const double f = mw_f(p, sh.ir[b][lane], sh.L[b][lane], c);
-  const double u = sh.u[b][lane];
-  if (warp == 0) return (u + f) * x;
-  if (warp == 1) return (u + f) * y;
-  return fma(sh.us[b][lane], sh.izb[b][lane], f) * z;
+  const double f = sh.A[lane] * fma(sh.L[lane], sh.ir[lane], -sh.inv_dh[lane]) + sh.B[lane];
+  if (warp < 2) return (sh.u[lane] + f) * q;
+  return fma(sh.us[lane], sh.izb[lane], f) * q;
 }
 
 __device__ __forceinline__ void team_write_save(const IntegrateArgs& a, const OrbitState& s, int64_t k, int j,
@@ -139,244 +158,245 @@ __device__ __forceinline__ void team_write_save(const IntegrateArgs& a, const Or
   a.out[j * a.out_stride + save_index(a, s, k)] = v;
 }
 
-// tqueue: the team's position counter; positions [0, min(tcap, *a.queue_len))
-// of a.order are the team's.
+// Takes queue positions [0, 16 gridDim.x) in stripes, then base +
+// atomicAdd(queue) (base: the positions that this launch and one running beside
+// it on the same queue hand out in stripes).
 template <class TB>
-__global__ void __launch_bounds__(128, 1) k_integrate_mw_team(IntegrateArgs a, MWParams p,
-                                                              unsigned long long* tqueue, long long tcap) {
+__global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, MWParams p, long long base) {
   constexpr int S = TB::S;
+  constexpr double kIdle = 8.0;  // position of lanes without an orbit
   __shared__ TeamShared sh;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = lane & (kTeamLanes - 1);
+  const bool hi = lane >= kTeamLanes;  // second stage of the pair
   const bool owner = warp < 3;
-  const int j0 = warp, j1 = warp + 3;  // owned components (warps 0-2)
-  const long long qlen = (long long)*a.queue_len;
-  const long long tlen = qlen < tcap ? qlen : tcap;
+  const int j0 = owner ? warp : 0, j1 = j0 + 3;  // owned components (warps 0-2)
+  const int jw = hi ? j1 : j0;                   // the one this lane writes out
+  const long long qlen = a.queue_len ? (long long)*a.queue_len : (long long)a.n;
   OrbitState s{};
   s.orbit = -1;
-  bool need_orbit = true, queue_open = true;
-  double yo0 = 0.0, yo1 = 0.0;  // owned state components j0, j1 (s.y holds all six for the controller)
-  double yn0 = 0.0, yn1 = 0.0;  // Dopri8: owned components of the accepted end state while saves are pending
-  double F0[2] = {0.0, 0.0};    // owned components of the slope at (tau, y)
-  bool need_f0 = false;         // Dopri8: the slope at a newly committed state is still to be evaluated
-  int round = 0;
+  bool need_orbit = true, queue_open = true, first = true;
+  double yp = 0.0, yv = 0.0;  // owned position and velocity component (s.y holds all six for the controller)
+  double np = 0.0, nv = 0.0;  // Dopri8: the same of the accepted end state while saves are pending
+  double F0v = 0.0;           // owned velocity component of the slope at (tau, y); its position component is yv
+  bool need_f0 = false;       // Dopri8: the slope at a newly committed state is still to be evaluated
   while (true) {
-    // ---- lanes without an orbit take the next queue position (warp 0 dequeues)
-    if (warp == 0 && need_orbit && queue_open) {
-      const unsigned long long k = atomicAdd(tqueue, 1ULL);
-      sh.slot[lane] = ((long long)k < tlen) ? (long long)a.order[k] : -1;
+    // ---- orbits for free lanes (warp 0 dequeues)
+    if (warp == 0 && !hi && need_orbit && queue_open) {
+      const long long k = first ? (long long)slot * gridDim.x + blockIdx.x : base + (long long)atomicAdd(a.queue, 1ULL);
+      sh.slot[slot] = k < qlen ? (a.order ? (long long)a.order[k] : k) : -1;
     }
+    first = false;
     __syncthreads();
     bool fresh = false;
     if (need_orbit && queue_open) {
-      const long long o = sh.slot[lane];
+      const long long o = sh.slot[slot];
       if (o < 0) {
         queue_open = false;
-      } else {  // resume a parked orbit (start_orbit, phase 1)
+      } else {
         s.orbit = o;
         const double t0 = a.t0[o], t1 = a.t1[o];
-        if (a.save_offsets) {
-          s.save_base = a.save_offsets[o];
-          s.save_end = a.save_offsets[o + 1] - s.save_base;
+        begin_orbit(a, s, t0, t1);
+        if (a.phase == 1) {
+          resume_orbit(a, s);
+          fresh = true;
         } else {
-          s.save_base = o;
-          s.save_end = a.n_saves;
+          const int32_t st = !isfinite(t0) || !isfinite(t1) ? ORBIT_NONFINITE : ORBIT_OK;
+          if (t0 == t1 || st != ORBIT_OK) {  // as start_orbit: nothing to integrate, or no end
+            if (warp == 0 && !hi) {
+              if (t0 == t1)
+                for (; s.save_i < s.save_end; ++s.save_i) write_save(a, s, s.save_i, s.y);
+              finish_orbit(a, s, t0 == t1 ? ORBIT_OK : st);
+            }
+            s.orbit = -1;
+          } else {
+            fresh = true;
+          }
         }
-        s.pending = 0;
-        s.dir = (t0 < t1) ? 1.0 : -1.0;
-        s.tau0 = s.dir * t0;
-        s.tau1 = s.dir * t1;
-        const OrbitResume& r = a.resume[o];
-#pragma unroll
-        for (int j = 0; j < 6; ++j) s.y[j] = r.y[j];
-        yo0 = r.y[j0 < 6 ? j0 : 0];
-        yo1 = r.y[j1 < 6 ? j1 : 0];
-        s.tau = r.tau;
-        s.tnext = r.tnext;
-        s.prev_inv = r.prev_inv;
-        s.prev_prev_inv = r.prev_prev_inv;
-        s.nsteps = r.nsteps;
-        s.naccepted = r.naccepted;
-        s.save_i = r.save_i;
-        s.at_dtmin = r.at_dtmin;
-        s.status = r.status;
-        fresh = true;
-        need_orbit = false;
+        if (fresh) {
+          yp = j0 == 0 ? s.y[0] : j0 == 1 ? s.y[1] : s.y[2];  // no dynamic index: s.y stays in registers
+          yv = j0 == 0 ? s.y[3] : j0 == 1 ? s.y[4] : s.y[5];
+          need_orbit = false;
+        }
       }
     }
     const bool active = s.orbit >= 0;
-    if (!__syncthreads_or(active)) break;
-    // ---- slope at resumed (and, for Dopri8, newly committed) states: one team
+    if (!__syncthreads_or(active)) {
+      if (!__syncthreads_or(need_orbit && queue_open)) break;
+      continue;
+    }
+    // ---- slope at new states (and, for Dopri8, newly committed ones): one
     // round, only when a lane needs it
     const bool want_f0 = fresh || (need_f0 && active);
     if (__syncthreads_or(want_f0)) {
-      const int b = round++ & 1;
-      if (owner) sh.pos[b][warp][lane] = want_f0 ? yo0 : 8.0;
-      const double g = team_grad(sh, b, warp, lane, p);
-      if (owner && want_f0) {
-        F0[0] = yo1;
-        F0[1] = -g;
-      }
+      const double g = team_grad(sh, warp, lane, p, want_f0 ? yp : kIdle);
+      if (want_f0) F0v = -g;
     }
     need_f0 = false;
+    // ---- first step of orbits that start here (start_orbit, initial_step)
+    const bool start = fresh && a.phase == 0;
+    const bool probe = start && a.adaptive && !(a.dt0 > 0.0);
+    double h_init = a.dt0;
+    if (__syncthreads_or(probe)) {
+      if (owner && !hi) {
+        sh.y1[j0][slot] = yv;
+        sh.y1[j1][slot] = F0v;
+      }
+      __syncthreads();
+      InitialStep is{};
+      double F0[6];
+#pragma unroll
+      for (int j = 0; j < 6; ++j) F0[j] = sh.y1[j][slot];
+      if (probe) is = initial_probe(a, s.y, F0);
+      const double g = team_grad(sh, warp, lane, p, probe ? fma(is.h0 * s.dir, yv, yp) : kIdle);
+      if (owner && !hi) {
+        sh.err[j0][slot] = fma(is.h0 * s.dir, F0v, yv);
+        sh.err[j1][slot] = -g;
+      }
+      __syncthreads();
+      if (probe) {
+        double F1[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) F1[j] = sh.err[j][slot];
+        h_init = initial_finish<TB>(is, F0, F1);
+      }
+    }
+    if (start) first_step(a, s, h_init);
     // ---- one RK evaluation (integrate_loop): a step from (tau, y), or for
     // Dopri8 with saves pending the sub-step from (tau, y) to the next save
     const bool sub = !TB::FSAL && s.pending && active;
     const double hs = sub ? s.dir * (save_tau(a, s, s.save_i) - s.tau) : s.dir * (s.tnext - s.tau);
-    double Fp[S], Fv[S];  // owned components of the stage slopes: position j0, velocity j1
-    Fp[0] = F0[0];
-    Fv[0] = F0[1];
-    static_for<1, S>([&](auto i) {
-      constexpr int I = decltype(i)::value;
-      const int b = round++ & 1;
-      double Yv = 0.0;
+    double Fp[S], Fv[S];  // owned components of the stage slopes: position, velocity
+    Fp[0] = yv;
+    Fv[0] = F0v;
+    double y1p = 0.0, y1v = 0.0;
+    static_for<0, (S - 1) / 2>([&](auto r) {
+      constexpr int I = 2 * decltype(r)::value + 1;  // stages I (lanes 0-15) and I + 1 (lanes 16-31)
+      double q = 0.0;
       if (owner) {
-        const double Yp = stage_comp<TB, I>(yo0, hs, Fp);
-        Yv = stage_comp<TB, I>(yo1, hs, Fv);
-        sh.pos[b][warp][lane] = active ? Yp : 8.0;
+        if constexpr (I == 1) {
+          Fp[1] = pair_row<TB, 1, 1>(hi, yv, hs, Fv);
+        } else {
+          const double V = pair_row<TB, I - 1, I>(hi, yv, hs, Fv);
+          const double W = __shfl_xor_sync(0xffffffffu, V, kTeamLanes);
+          Fp[I - 1] = hi ? W : V;
+          Fp[I] = hi ? V : W;
+        }
+        q = pair_row<TB, I, I + 1>(hi, yp, hs, Fp);
       }
-      const double g = team_grad(sh, b, warp, lane, p);
-      Fp[I] = Yv;
-      Fv[I] = -g;
+      const double f = -team_grad(sh, warp, lane, p, active ? q : kIdle);
+      const double o = __shfl_xor_sync(0xffffffffu, f, kTeamLanes);
+      Fv[I] = hi ? o : f;
+      Fv[I + 1] = hi ? f : o;
+      if constexpr (TB::FSAL && I + 2 == S) y1p = q;  // the last row is the solution's (lanes 16-31)
     });
     // solution and error for the owned components, then the shared controller
-    double y1o0 = 0.0, y1o1 = 0.0;
     if (owner) {
-      y1o0 = weighted_comp<TB, W_SOLUTION, true>(yo0, hs, Fp);
-      y1o1 = weighted_comp<TB, W_SOLUTION, true>(yo1, hs, Fv);
-      sh.y1[j0][lane] = y1o0;
-      sh.y1[j1][lane] = y1o1;
-      if (a.adaptive && !sub) {
-        sh.err[j0][lane] = weighted_comp<TB, W_ERROR, false>(0.0, hs, Fp);
-        sh.err[j1][lane] = weighted_comp<TB, W_ERROR, false>(0.0, hs, Fv);
+      const bool want_err = a.adaptive && !sub;
+      Fp[S - 1] = pair_row<TB, S - 1, S - 1>(hi, yv, hs, Fv);
+      if constexpr (TB::FSAL) {
+        y1v = Fp[S - 1];
+        const double other = __shfl_xor_sync(0xffffffffu, y1p, kTeamLanes);
+        y1p = hi ? y1p : other;
+      } else {
+        y1p = weighted_comp<TB, W_SOLUTION, true>(yp, hs, Fp);
+        y1v = weighted_comp<TB, W_SOLUTION, true>(yv, hs, Fv);
+      }
+      sh.y1[jw][slot] = hi ? y1v : y1p;
+      if (want_err) {
+        double Fw[S];
+#pragma unroll
+        for (int l = 0; l < S; ++l) Fw[l] = hi ? Fv[l] : Fp[l];
+        sh.err[jw][slot] = weighted_comp<TB, W_ERROR, false>(0.0, hs, Fw);
       }
     }
     __syncthreads();
     double y1[6], err[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
-      y1[j] = sh.y1[j][lane];
-      err[j] = a.adaptive ? sh.err[j][lane] : 0.0;
+      y1[j] = sh.y1[j][slot];
+      err[j] = a.adaptive ? sh.err[j][slot] : 0.0;
     }
     __syncthreads();  // the exchange arrays are reused next step
     if (!active) continue;
-    if constexpr (!TB::FSAL) {
-      if (sub) {  // the partial step's end is a save of the accepted step
-        if (owner) {
-          team_write_save(a, s, s.save_i, j0, y1o0);
-          team_write_save(a, s, s.save_i, j1, y1o1);
-        }
-        ++s.save_i;
-        if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= s.tau_new) continue;
-        // all saves of the accepted step written: commit it
-        s.pending = 0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) s.y[j] = s.ynew[j];
-        yo0 = yn0;
-        yo1 = yn1;
-        s.tau = fmin(s.tau_new, s.tau1);
-        need_f0 = true;
-        s.tnext = s.tnext_new;
-        bool done = false;
-        int32_t st = ORBIT_OK;
-        if (s.status != ORBIT_OK) {
-          done = true;
-          st = s.status;
-        } else if (s.tau >= s.tau1) {
-          done = true;
-        } else if (s.nsteps >= a.max_steps) {
-          done = true;
-          st = ORBIT_MAX_STEPS;
-        }
-        if (done) {
-          if (warp == 0) {
-            finish_orbit(a, s, st);
-          } else {
-            s.orbit = -1;
-          }
-          need_orbit = true;
-          need_f0 = false;
-        }
-        continue;
-      }
-    }
-    ++s.nsteps;
-    const double h = s.tnext - s.tau;
-    double next_t0, next_t1;
-    bool keep;
-    if (a.adaptive) {
-      keep = pid_adapt<TB::ORDER>(a, s, y1, err, h, next_t0, next_t1);
-    } else {
-      keep = true;
-      next_t0 = s.tnext;
-      next_t1 = s.tnext + a.dt0;
-    }
-    bool finite = true;
-#pragma unroll
-    for (int j = 0; j < 6; ++j) finite = finite && isfinite(y1[j]);
     bool done = false;
     int32_t st = ORBIT_OK;
-    if (!finite) {
-      done = true;
-      st = ORBIT_NONFINITE;
+    if (sub) {  // the partial step's end is a save of the accepted step
+      if (owner) team_write_save(a, s, s.save_i, jw, hi ? y1v : y1p);
+      ++s.save_i;
+      if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= s.tau_new) continue;
+      // all saves of the accepted step written: commit it
+      s.pending = 0;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) s.y[j] = s.ynew[j];
+      yp = np;
+      yv = nv;
+      s.tau = fmin(s.tau_new, s.tau1);
+      need_f0 = true;
+      s.tnext = s.tnext_new;
     } else {
-      const double tprev_new = fmin(next_t0, s.tau1);
-      const double tnext_new = clip_to_end(tprev_new, next_t1, s.tau1, keep);
-      if (keep) {
-        ++s.naccepted;
-        if constexpr (TB::FSAL) {
-          if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
-            const double ih = 1.0 / h;
-            do {
-              const double th = (save_tau(a, s, s.save_i) - s.tau) * ih;
-              if (owner) {
-                team_write_save(a, s, s.save_i, j0, dense_comp(yo0, hs, Fp, th));
-                team_write_save(a, s, s.save_i, j1, dense_comp(yo1, hs, Fv, th));
-              }
-              ++s.save_i;
-            } while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0);
-          }
-#pragma unroll
-          for (int j = 0; j < 6; ++j) s.y[j] = y1[j];
-          yo0 = y1o0;
-          yo1 = y1o1;
-          F0[0] = Fp[S - 1];
-          F0[1] = Fv[S - 1];
-          s.tau = tprev_new;
-          s.tnext = tnext_new;
-        } else {
-          if (a.defer != nullptr) {
-            while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
-              const bool at_end = save_tau(a, s, s.save_i) == s.tnext;  // as put_deferred_save
-              if (owner) {
-                team_write_save(a, s, s.save_i, j0, at_end ? y1o0 : yo0);
-                team_write_save(a, s, s.save_i, j1, at_end ? y1o1 : yo1);
-              }
-              if (warp == 3 && !at_end) a.defer[save_index(a, s, s.save_i)] = s.dir * s.tau;
-              ++s.save_i;
-            }
-          } else if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
-            // saves inside this step: keep (tau, y) for the sub-steps
-            s.pending = 1;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) s.ynew[j] = y1[j];
-            yn0 = y1o0;
-            yn1 = y1o1;
-            s.tau_new = next_t0;
-            s.tnext_new = tnext_new;
-            continue;
-          }
-#pragma unroll
-          for (int j = 0; j < 6; ++j) s.y[j] = y1[j];
-          yo0 = y1o0;
-          yo1 = y1o1;
-          s.tau = tprev_new;
-          s.tnext = tnext_new;
-          need_f0 = true;
-        }
+      ++s.nsteps;
+      const double h = s.tnext - s.tau;
+      double next_t0, next_t1;
+      bool keep;
+      if (a.adaptive) {
+        keep = pid_adapt<TB::ORDER>(a, s, y1, err, h, next_t0, next_t1);
       } else {
+        keep = true;
+        next_t0 = s.tnext;
+        next_t1 = s.tnext + a.dt0;
+      }
+      bool finite = true;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) finite = finite && isfinite(y1[j]);
+      if (!finite) {
+        done = true;
+        st = ORBIT_NONFINITE;
+      } else {
+        const double tprev_new = fmin(next_t0, s.tau1);
+        const double tnext_new = clip_to_end(tprev_new, next_t1, s.tau1, keep);
+        if (keep) {
+          ++s.naccepted;
+          if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+            if constexpr (TB::FSAL) {
+              const double ih = 1.0 / h;
+              double Fw[S];
+#pragma unroll
+              for (int l = 0; l < S; ++l) Fw[l] = hi ? Fv[l] : Fp[l];
+              do {
+                const double th = (save_tau(a, s, s.save_i) - s.tau) * ih;
+                if (owner) team_write_save(a, s, s.save_i, jw, dense_comp(hi ? yv : yp, hs, Fw, th));
+                ++s.save_i;
+              } while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0);
+            } else if (a.defer != nullptr) {
+              do {
+                const bool at_end = save_tau(a, s, s.save_i) == s.tnext;  // as put_deferred_save
+                if (owner) team_write_save(a, s, s.save_i, jw, at_end ? (hi ? y1v : y1p) : (hi ? yv : yp));
+                if (warp == 3 && !hi && !at_end) a.defer[save_index(a, s, s.save_i)] = s.dir * s.tau;
+                ++s.save_i;
+              } while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0);
+            } else {  // saves inside this step: keep (tau, y) for the sub-steps
+              s.pending = 1;
+#pragma unroll
+              for (int j = 0; j < 6; ++j) s.ynew[j] = y1[j];
+              np = y1p;
+              nv = y1v;
+              s.tau_new = next_t0;
+              s.tnext_new = tnext_new;
+              continue;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 6; ++j) s.y[j] = y1[j];
+          yp = y1p;
+          yv = y1v;
+          if constexpr (TB::FSAL) F0v = Fv[S - 1];
+          need_f0 = !TB::FSAL;
+        }
         s.tau = tprev_new;
         s.tnext = tnext_new;
       }
+    }
+    if (!done) {
       if (s.status != ORBIT_OK) {
         done = true;
         st = s.status;
@@ -388,11 +408,8 @@ __global__ void __launch_bounds__(128, 1) k_integrate_mw_team(IntegrateArgs a, M
       }
     }
     if (done) {
-      if (warp == 0) {
-        finish_orbit(a, s, st);
-      } else {
-        s.orbit = -1;
-      }
+      if (warp == 0 && !hi) finish_orbit(a, s, st);
+      s.orbit = -1;
       need_orbit = true;
       need_f0 = false;
     }

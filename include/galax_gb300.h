@@ -257,13 +257,14 @@ GAL_API gal_status gal_dense_evaluate(const gal_potential* pot, int32_t method, 
  * threads at maximum occupancy (variant 0 for Dopri5, 2 for Dopri8). */
 GAL_API gal_status gal_set_launch(int32_t method, int32_t adaptive, int32_t block_threads, int32_t blocks_per_sm,
                                   int32_t variant);
-/* Second pass of a two-pass Dopri5 or Dopri8 batch in the Milky Way model: `blocks` > 0
- * (default 32, at most the SM count - 1) hands the 32 x blocks longest orbits to
- * four-warp team blocks, each on an SM of its own, on a library-owned stream
- * beside the one-thread-per-orbit kernel, which runs one block per remaining
- * SM; 0 keeps every orbit on the one-thread kernel with the launch shape of
- * gal_set_launch. Results are bitwise identical either way; the teams cut the
- * serial latency of the longest orbits. Process-wide. */
+/* Four-warp team blocks (16 orbits each, two Runge-Kutta stages per round) in
+ * the Milky Way model. blocks > 0 (default 32, at most the SM count - 1): small
+ * batches run on teams alone, and the second pass of a larger two-pass batch
+ * gives `blocks` SMs to teams, which take the longest orbits first, on a
+ * library-owned stream beside the one-thread-per-orbit kernel, which runs one
+ * block per remaining SM. 0 keeps every orbit on the one-thread kernel with the
+ * launch shape of gal_set_launch. Results are bitwise identical either way; the
+ * teams cut the serial latency of few or long orbits. Process-wide. */
 GAL_API gal_status gal_set_team(int32_t blocks);
 /* Fraction of every orbit's span that the first pass of the two-pass schedule
  * (cfg->schedule = 1) covers before the orbits are ordered by their remaining
