@@ -36,6 +36,45 @@ namespace gal {
 
 enum { ORBIT_OK = 0, ORBIT_MAX_STEPS = 1, ORBIT_DT_MIN = 2, ORBIT_NONFINITE = 3 };
 
+// Comparisons, sign changes and finiteness tests on the bits, in integer
+// registers. On GB300 an FP64 comparison, minimum or maximum occupies the FP64
+// pipe like an arithmetic instruction (and takes ~110 cycles to return), while
+// a two-word integer comparison takes a few; a step's control has about forty
+// of them. The results are those of the FP64 operations they stand for.
+__device__ __forceinline__ long long dbits(double v) { return __double_as_longlong(v); }
+constexpr long long kInfBits = 0x7FF0000000000000LL;
+__device__ __forceinline__ bool bits_finite(double v) { return (__double2hiint(v) & 0x7FF00000) != 0x7FF00000; }
+__device__ __forceinline__ bool bits_nan(double v) { return (dbits(v) & 0x7FFFFFFFFFFFFFFFLL) > kInfBits; }
+// v > 0 (false for NaN)
+__device__ __forceinline__ bool gt_zero(double v) { return dbits(v) > 0 && dbits(v) <= kInfBits; }
+// v with the sign of s * v, s = +-1
+__device__ __forceinline__ double with_sign(double s, double v) {
+  return __hiloint2double(__double2hiint(v) ^ (__double2hiint(s) & 0x80000000), __double2loint(v));
+}
+// integers in the order of the numbers (-0 just below +0)
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = dbits(v);
+  return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL);
+}
+// a <= b and a < b for b not NaN; false where a is NaN. Zeros of either sign are equal.
+__device__ __forceinline__ bool le_bits(double a, double b) {
+  return !bits_nan(a) && (order_key(a) <= order_key(b) || ((dbits(a) | dbits(b)) & 0x7FFFFFFFFFFFFFFFLL) == 0);
+}
+__device__ __forceinline__ bool lt_bits(double a, double b) { return !bits_nan(a) && !le_bits(b, a); }
+// smaller and larger of two numbers that are not negative and not NaN
+__device__ __forceinline__ double min_pos(double a, double b) { return dbits(a) < dbits(b) ? a : b; }
+__device__ __forceinline__ double max_pos(double a, double b) { return dbits(a) > dbits(b) ? a : b; }
+
+// a / 6 correctly rounded for 1e-250 < a < 1e250 (a > 0): the product with the
+// rounded 1/6 and one correction by its exact residual (P. W. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34(1), 1990); three FP64 instructions instead of a division.
+__device__ __forceinline__ double sixth(double a) {
+  constexpr double y = 1.0 / 6.0;
+  const double q = a * y;
+  return fma(fma(-6.0, q, a), y, q);
+}
+
 constexpr int kTeamLanes = 16;  // orbits per four-warp team block (integrate_team.cuh)
 
 // Everything needed to continue an orbit exactly where a first pass parked it
@@ -236,7 +275,7 @@ __device__ __forceinline__ void write_save(const IntegrateArgs& a, const OrbitSt
 
 __device__ __forceinline__ double save_tau(const IntegrateArgs& a, const OrbitState& s, int64_t k) {
   const double ts = a.save_offsets ? a.save_ts[s.save_base + k] : a.save_ts[k];
-  return s.dir * ts;
+  return with_sign(s.dir, ts);
 }
 
 // Dopri8 saves are partial steps of their own from the start of the step they
@@ -253,10 +292,10 @@ __device__ __forceinline__ double save_tau(const IntegrateArgs& a, const OrbitSt
 __device__ __forceinline__ void put_deferred_save(const IntegrateArgs& a, const OrbitState& s, double tau_k,
                                                   const double* y1) {
   const int64_t idx = save_index(a, s, s.save_i);
-  const bool at_end = tau_k == s.tnext;
+  const bool at_end = dbits(tau_k) == dbits(s.tnext);
 #pragma unroll
   for (int j = 0; j < 6; ++j) a.out[j * a.out_stride + idx] = at_end ? y1[j] : s.y[j];
-  if (!at_end) a.defer[idx] = s.dir * s.tau;
+  if (!at_end) a.defer[idx] = with_sign(s.dir, s.tau);
 }
 
 __device__ __forceinline__ void finish_orbit(const IntegrateArgs& a, OrbitState& s, int32_t st) {
@@ -441,10 +480,10 @@ __device__ __forceinline__ bool start_orbit(const IntegrateArgs& a, const Pot& p
 // Phase 0 of the two-phase schedule: park the orbit once it has covered
 // split_frac of its span (only between steps, never with saves pending).
 __device__ __forceinline__ bool maybe_park(const IntegrateArgs& a, OrbitState& s) {
-  if (a.phase != 0 || a.split_frac <= 0.0) return false;
+  if (a.phase != 0 || !gt_zero(a.split_frac)) return false;
   const double span = s.tau1 - s.tau0;
   const double done = s.tau - s.tau0;
-  if (done < a.split_frac * span) return false;
+  if (lt_bits(done, a.split_frac * span)) return false;
   OrbitResume& r = a.resume[s.orbit];
 #pragma unroll
   for (int j = 0; j < 6; ++j) r.y[j] = s.y[j];
@@ -496,14 +535,14 @@ __device__ __forceinline__ bool pid_adapt(const IntegrateArgs& a, OrbitState& s,
   double d[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    const double y1c = isnan(y1[j]) ? s.y[j] : y1[j];
-    d[j] = fma(fmax(fabs(s.y[j]), fabs(y1c)), a.rtol, a.atol);
+    const double y0c = fabs(s.y[j]), y1c = bits_nan(y1[j]) ? y0c : fabs(y1[j]);
+    d[j] = fma(max_pos(y0c, y1c), a.rtol, a.atol);
   }
   const double p01 = d[0] * d[1], p23 = d[2] * d[3], p45 = d[4] * d[5];
   const double p0123 = p01 * p23;
   const double P = p0123 * p45;
   double ms = 0.0;
-  if (P > 1e-280 && P < 1e280) {
+  if (dbits(P) > dbits(1e-280) && dbits(P) < dbits(1e280)) {
     const double iP = 1.0 / P;
     const double i01 = iP * p23 * p45, i23 = iP * p01 * p45, i45 = iP * p0123;
     const double r[6] = {i01 * d[1], i01 * d[0], i23 * d[3], i23 * d[2], i45 * d[5], i45 * d[4]};
@@ -519,14 +558,17 @@ __device__ __forceinline__ bool pid_adapt(const IntegrateArgs& a, OrbitState& s,
       ms = fma(q, q, ms);
     }
   }
-  ms = ms / 6.0;
-  bool keep = ms < 1.0;  // scaled error = sqrt(ms) < 1
-  if (a.dtmin > 0.0) keep = keep || s.at_dtmin;
+  // ms >= 0 or NaN, whose bits as an unsigned number are above all others'
+  const unsigned long long um = (unsigned long long)dbits(ms);
+  ms = um > (unsigned long long)dbits(1e-250) && um < (unsigned long long)dbits(1e250) ? sixth(ms) : ms / 6.0;
+  const unsigned long long ub = (unsigned long long)dbits(ms);
+  bool keep = ub < (unsigned long long)dbits(1.0);  // scaled error = sqrt(ms) < 1
+  if (gt_zero(a.dtmin)) keep = keep || s.at_dtmin;
   const double fmin_ = keep ? 1.0 : a.factormin;
   double factor;
-  if (a.i_controller && ms >= 1e-30 && ms <= 1e30) {
+  if (a.i_controller && ub >= (unsigned long long)dbits(1e-30) && ub <= (unsigned long long)dbits(1e30)) {
     // integral controller: factor = safety * (1/scaled)^(1/order) = safety * ms^(-1/(2 order))
-    factor = fmin(fmax(a.safety * inv_root<ORDER>(ms), fmin_), a.factormax);
+    factor = min_pos(max_pos(a.safety * inv_root<ORDER>(ms), fmin_), a.factormax);
   } else {
     double inv = 1.0 / sqrt(ms);
     const double f1 = (a.c1 == 0.0) ? 1.0 : pow(inv, a.c1);
@@ -540,8 +582,8 @@ __device__ __forceinline__ bool pid_adapt(const IntegrateArgs& a, OrbitState& s,
     }
   }
   double dt = h * factor;
-  if (a.dtmax > 0.0) dt = fmin(dt, a.dtmax);
-  if (a.dtmin > 0.0) {
+  if (gt_zero(a.dtmax)) dt = fmin(dt, a.dtmax);
+  if (gt_zero(a.dtmin)) {
     if (!a.force_dtmin && dt < a.dtmin) s.status = ORBIT_DT_MIN;
     s.at_dtmin = dt <= a.dtmin;
     dt = fmax(dt, a.dtmin);
@@ -551,9 +593,14 @@ __device__ __forceinline__ bool pid_adapt(const IntegrateArgs& a, OrbitState& s,
   return keep;
 }
 
+// min(next_t0, tau1), the start of the next step
+__device__ __forceinline__ double clip_start(double next_t0, double tau1) {
+  return lt_bits(tau1, next_t0) ? tau1 : next_t0;
+}
+
 __device__ __forceinline__ double clip_to_end(double tprev, double tnext, double tau1, bool keep) {
   // diffrax _clip_to_end: float64 tolerance 1e-10
-  if (tnext > tau1 - 1e-10) return keep ? tau1 : tprev + 0.5 * (tau1 - tprev);
+  if (lt_bits(tau1 - 1e-10, tnext)) return keep ? tau1 : tprev + 0.5 * (tau1 - tprev);
   return tnext;
 }
 
@@ -573,13 +620,13 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
     // for Dopri8, the sub-step from (tau, y) to a save time of the step just accepted.
     double hs;
     if (TB::FSAL || !s.pending) {
-      hs = s.dir * (s.tnext - s.tau);
+      hs = with_sign(s.dir, s.tnext - s.tau);
     } else {
-      hs = s.dir * (save_tau(a, s, s.save_i) - s.tau);
+      hs = with_sign(s.dir, save_tau(a, s, s.save_i) - s.tau);
     }
 #pragma unroll
     for (int j = 0; j < 6; ++j) F[0][j] = s.F0[j];
-    rk_stages<TB>(pot, s.y, hs, F, s.dir * s.tau);
+    rk_stages<TB>(pot, s.y, hs, F, with_sign(s.dir, s.tau));
     double y1[6], err[6];
     int32_t st = ORBIT_OK;
     bool done = false;
@@ -587,16 +634,16 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
       rk_combine<TB>(s.y, hs, F, y1, nullptr);
       write_save(a, s, s.save_i, y1);
       ++s.save_i;
-      if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= s.tau_new) continue;
+      if (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), s.tau_new)) continue;
       // all saves of the accepted step written: commit it
       s.pending = 0;
 #pragma unroll
       for (int j = 0; j < 6; ++j) s.y[j] = s.ynew[j];
-      s.tau = fmin(s.tau_new, s.tau1);
-      field(pot, s.y, s.F0, s.dir * s.tau);
+      s.tau = clip_start(s.tau_new, s.tau1);
+      field(pot, s.y, s.F0, with_sign(s.dir, s.tau));
       s.tnext = s.tnext_new;
       if (s.status != ORBIT_OK) { done = true; st = s.status; }
-      else if (s.tau >= s.tau1) done = true;
+      else if (le_bits(s.tau1, s.tau)) done = true;
       else if (s.nsteps >= a.max_steps) { done = true; st = ORBIT_MAX_STEPS; }
       else if (maybe_park(a, s)) {
         if (!start_orbit<TB, Pot, LANES>(a, pot, s, first)) return;
@@ -617,18 +664,18 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
       }
       bool finite = true;
 #pragma unroll
-      for (int j = 0; j < 6; ++j) finite = finite && isfinite(y1[j]);
+      for (int j = 0; j < 6; ++j) finite = finite && bits_finite(y1[j]);
       if (!finite) {
         done = true;
         st = ORBIT_NONFINITE;
       } else {
-        const double tprev_new = fmin(next_t0, s.tau1);
+        const double tprev_new = clip_start(next_t0, s.tau1);
         const double tnext_new = clip_to_end(tprev_new, next_t1, s.tau1, keep);
         if (keep) {
           ++s.naccepted;
           if constexpr (TB::FSAL) {
             // Dopri5: saves in (tau, tnext] from the quartic dense output
-            if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+            if (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0)) {
               const double ih = 1.0 / h;
               do {
                 const double th = (save_tau(a, s, s.save_i) - s.tau) * ih;
@@ -636,7 +683,7 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
                 dopri5_dense(s.y, hs, F, th, v);
                 write_save(a, s, s.save_i, v);
                 ++s.save_i;
-              } while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0);
+              } while (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0));
             }
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
@@ -647,11 +694,11 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
             s.tnext = tnext_new;
           } else {
             if (a.defer != nullptr) {
-              while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+              while (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0)) {
                 put_deferred_save(a, s, save_tau(a, s, s.save_i), y1);
                 ++s.save_i;
               }
-            } else if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+            } else if (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0)) {
               // Dopri8 with saves inside this step: keep (tau, y) for the sub-steps
               s.pending = 1;
 #pragma unroll
@@ -664,14 +711,14 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
             for (int j = 0; j < 6; ++j) s.y[j] = y1[j];
             s.tau = tprev_new;
             s.tnext = tnext_new;
-            field(pot, s.y, s.F0, s.dir * s.tau);
+            field(pot, s.y, s.F0, with_sign(s.dir, s.tau));
           }
         } else {
           s.tau = tprev_new;
           s.tnext = tnext_new;
         }
         if (s.status != ORBIT_OK) { done = true; st = s.status; }
-        else if (s.tau >= s.tau1) done = true;
+        else if (le_bits(s.tau1, s.tau)) done = true;
         else if (s.nsteps >= a.max_steps) { done = true; st = ORBIT_MAX_STEPS; }
         else if (maybe_park(a, s)) {
           if (!start_orbit<TB, Pot, LANES>(a, pot, s, first)) return;

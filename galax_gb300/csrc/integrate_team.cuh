@@ -52,27 +52,24 @@ struct TeamShared {
   long long slot[kTeamLanes];
 };
 
-// One coefficient of each half of the lanes; zero coefficients add nothing, as
-// in stage_state, where their terms do not exist.
-template <bool FIRST>
-__device__ __forceinline__ double pair_term(bool hi, double ca, double cb, double F, double acc) {
-  const double c = hi ? cb : ca;
-  if constexpr (FIRST) return c * F;
-  const double t = fma(c, F, acc);
-  if (ca != 0.0 && cb != 0.0) return t;
-  return (hi ? cb : ca) != 0.0 ? t : acc;
-}
-
 // Y_j = y_j + hs sum_{l<I} A[I][l] F_l,j for one component (stage_state's
-// arithmetic): row IA on lanes 0-15, row IB on lanes 16-31.
+// arithmetic): row IA on lanes 0-15, row IB on lanes 16-31. Zero coefficients
+// add nothing, as in stage_state, where their terms do not exist.
 template <class TB, int IA, int IB>
 __device__ __forceinline__ double pair_row(bool hi, double yj, double hs, const double (&Fj)[TB::S]) {
   static_assert(TB::A[IA][0] != 0.0 && TB::A[IB][0] != 0.0, "rows start with their first slope");
-  double acc = pair_term<true>(hi, TB::A[IA][0], TB::A[IB][0], Fj[0], 0.0);
+  constexpr double a0 = TB::A[IA][0], b0 = TB::A[IB][0];
+  double acc = (hi ? b0 : a0) * Fj[0];
   static_for<1, (IA > IB ? IA : IB)>([&](auto l) {
     constexpr int L = decltype(l)::value;
     constexpr double ca = L < IA ? TB::A[IA][L] : 0.0, cb = L < IB ? TB::A[IB][L] : 0.0;
-    if constexpr (ca != 0.0 || cb != 0.0) acc = pair_term<false>(hi, ca, cb, Fj[L], acc);
+    if constexpr (ca != 0.0 || cb != 0.0) {
+      constexpr double sa = ca != 0.0 ? ca : cb, sb = cb != 0.0 ? cb : ca;
+      const double t = fma(hi ? sb : sa, Fj[L], acc);
+      if constexpr (ca == 0.0) acc = hi ? t : acc;
+      else if constexpr (cb == 0.0) acc = hi ? acc : t;
+      else acc = t;
+    }
   });
   return fma(hs, acc, yj);
 }
@@ -234,7 +231,7 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
     need_f0 = false;
     // ---- first step of orbits that start here (start_orbit, initial_step)
     const bool start = fresh && a.phase == 0;
-    const bool probe = start && a.adaptive && !(a.dt0 > 0.0);
+    const bool probe = start && a.adaptive && !gt_zero(a.dt0);
     double h_init = a.dt0;
     if (__syncthreads_or(probe)) {
       if (owner && !hi) {
@@ -264,7 +261,7 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
     // ---- one RK evaluation (integrate_loop): a step from (tau, y), or for
     // Dopri8 with saves pending the sub-step from (tau, y) to the next save
     const bool sub = !TB::FSAL && s.pending && active;
-    const double hs = sub ? s.dir * (save_tau(a, s, s.save_i) - s.tau) : s.dir * (s.tnext - s.tau);
+    const double hs = with_sign(s.dir, (sub ? save_tau(a, s, s.save_i) : s.tnext) - s.tau);
     double Fp[S], Fv[S];  // owned components of the stage slopes: position, velocity
     Fp[0] = yv;
     Fv[0] = F0v;
@@ -323,14 +320,14 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
     if (sub) {  // the partial step's end is a save of the accepted step
       if (owner) team_write_save(a, s, s.save_i, jw, hi ? y1v : y1p);
       ++s.save_i;
-      if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= s.tau_new) continue;
+      if (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), s.tau_new)) continue;
       // all saves of the accepted step written: commit it
       s.pending = 0;
 #pragma unroll
       for (int j = 0; j < 6; ++j) s.y[j] = s.ynew[j];
       yp = np;
       yv = nv;
-      s.tau = fmin(s.tau_new, s.tau1);
+      s.tau = clip_start(s.tau_new, s.tau1);
       need_f0 = true;
       s.tnext = s.tnext_new;
     } else {
@@ -347,16 +344,16 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
       }
       bool finite = true;
 #pragma unroll
-      for (int j = 0; j < 6; ++j) finite = finite && isfinite(y1[j]);
+      for (int j = 0; j < 6; ++j) finite = finite && bits_finite(y1[j]);
       if (!finite) {
         done = true;
         st = ORBIT_NONFINITE;
       } else {
-        const double tprev_new = fmin(next_t0, s.tau1);
+        const double tprev_new = clip_start(next_t0, s.tau1);
         const double tnext_new = clip_to_end(tprev_new, next_t1, s.tau1, keep);
         if (keep) {
           ++s.naccepted;
-          if (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0) {
+          if (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0)) {
             if constexpr (TB::FSAL) {
               const double ih = 1.0 / h;
               double Fw[S];
@@ -366,14 +363,14 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
                 const double th = (save_tau(a, s, s.save_i) - s.tau) * ih;
                 if (owner) team_write_save(a, s, s.save_i, jw, dense_comp(hi ? yv : yp, hs, Fw, th));
                 ++s.save_i;
-              } while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0);
+              } while (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0));
             } else if (a.defer != nullptr) {
               do {
-                const bool at_end = save_tau(a, s, s.save_i) == s.tnext;  // as put_deferred_save
+                const bool at_end = dbits(save_tau(a, s, s.save_i)) == dbits(s.tnext);  // as put_deferred_save
                 if (owner) team_write_save(a, s, s.save_i, jw, at_end ? (hi ? y1v : y1p) : (hi ? yv : yp));
-                if (warp == 3 && !hi && !at_end) a.defer[save_index(a, s, s.save_i)] = s.dir * s.tau;
+                if (warp == 3 && !hi && !at_end) a.defer[save_index(a, s, s.save_i)] = with_sign(s.dir, s.tau);
                 ++s.save_i;
-              } while (s.save_i < s.save_end && save_tau(a, s, s.save_i) <= next_t0);
+              } while (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0));
             } else {  // saves inside this step: keep (tau, y) for the sub-steps
               s.pending = 1;
 #pragma unroll
@@ -400,7 +397,7 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
       if (s.status != ORBIT_OK) {
         done = true;
         st = s.status;
-      } else if (s.tau >= s.tau1) {
+      } else if (le_bits(s.tau1, s.tau)) {
         done = true;
       } else if (s.nsteps >= a.max_steps) {
         done = true;

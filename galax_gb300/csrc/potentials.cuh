@@ -31,23 +31,37 @@ enum Kind : int32_t { KEPLER = 0, HERNQUIST = 1, MIYAMOTO_NAGAI = 2, NFW = 3, PL
 
 constexpr double TINY = 2.2250738585072014e-308;  // DBL_MIN, galax's safe_sqrt offset
 
+// (double)k for |k| < 2^20 in integer registers: the leading one becomes the
+// implicit bit, the rest the top of the mantissa's high word.
+__device__ __forceinline__ double small_int_to_double(int k) {
+  const unsigned a = (unsigned)(k < 0 ? -k : k);
+  const int e = 31 - __clz((int)a);
+  const unsigned hi = (((unsigned)(1023 + e) << 20) | ((a << (20 - e)) & 0xFFFFFu)) | (k < 0 ? 0x80000000u : 0u);
+  return __hiloint2double(a != 0u ? (int)hi : 0, 0);
+}
+
 // log(1 + u) for u >= 0 (the NFW halo's log(1 + r / r_s)) by Tang's
 // table-driven method (P. T. P. Tang, "Table-driven implementation of the
 // logarithm function in IEEE floating-point arithmetic", ACM TOMS 16(4), 1990):
 // 1 + u = 2^k F_j (1 + r) with F_j = 1 + j/128 the nearest table point, so
 // |r| <= 1/256; log(F_j) is tabulated as hi + lo and log(1 + r) is its Taylor
 // polynomial to r^7 (truncation below 2e-18 relative). The rounding error of
-// 1 + u is folded into r. About 20 FP64 operations, where a lone FP64 chain
-// pays ~64 cycles for each; within ~1 unit in the last place.
+// 1 + u is folded into r. What is not arithmetic (the larger summand, F_j, the
+// exponent as a number) is put together from the bits in integer registers: a
+// lone FP64 chain pays ~64 cycles for each FP64 instruction, comparisons and
+// conversions included (17 instructions; 26 with those on the FP64 pipe).
+// Within ~1 unit in the last place.
 __device__ __forceinline__ double log1p_pos(double u) {
   const double x = 1.0 + u;
-  const double c = (u <= 1.0) ? u - (x - 1.0) : 1.0 - (x - u);  // x + c = 1 + u exactly
+  const bool small = __double_as_longlong(u) <= 0x3FF0000000000000LL;  // u <= 1
+  const double big = small ? 1.0 : u, tiny = small ? u : 1.0;
+  const double c = tiny - (x - big);  // x + c = 1 + u exactly
   const long long bits = __double_as_longlong(x);
   const int k = (int)(bits >> 52) - 1023;
   const long long mant = bits & 0x000FFFFFFFFFFFFFLL;
   const double m = __longlong_as_double(mant | 0x3FF0000000000000LL);  // x = 2^k m, 1 <= m < 2
   const int j = (int)((mant + (1LL << 44)) >> 45);                      // nearest j / 128, 0..128
-  const double F = 1.0 + (double)j * 0.0078125;                         // exact
+  const double F = __longlong_as_double(0x3FF0000000000000LL + ((long long)j << 45));      // 1 + j / 128
   const double scale = __longlong_as_double((long long)(1023 - k) << 52);  // 2^-k
   const double r = fma(c, scale, m - F) * __ldg(&kLogTable[j][0]);       // m - F is exact
   double q = fma(0.14285714285714285, r, -0.16666666666666666);
@@ -56,7 +70,7 @@ __device__ __forceinline__ double log1p_pos(double u) {
   q = fma(q, r, 0.3333333333333333);
   q = fma(q, r, -0.5);
   const double p = fma(r * r, q, r);
-  const double dk = (double)k;
+  const double dk = small_int_to_double(k);
   const double hi = fma(dk, 0.6931471805599453, __ldg(&kLogTable[j][1]));   // ln 2 = hi + lo
   const double lo = fma(dk, 2.3190468138462996e-17, __ldg(&kLogTable[j][2]));
   return hi + (lo + p);
@@ -514,8 +528,9 @@ __device__ __forceinline__ MWDisk mw_disk(const MWParams& p, double x, double y,
 }
 // centred spheres: 1/r and r
 __device__ __forceinline__ double mw_ir(double x, double y, double z, double& r) {
-  const double R2 = fma(x, x, y * y);
-  const double r2 = fma(z, z, R2 + TINY);
+  double R2 = fma(x, x, y * y);
+  if (__double2hiint(R2) < 0x06000000) R2 += TINY;  // changes nothing above 1e-280
+  const double r2 = fma(z, z, R2);
   const double ir = rsqrt(r2);
   r = r2 * ir;
   return ir;
