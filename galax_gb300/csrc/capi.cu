@@ -19,63 +19,13 @@
 namespace gal {
 
 thread_local std::string g_last_error;
-// SMs given to four-warp teams for the longest orbits (gal_set_team); atomic
-// because calls on other threads may read it while it is set
-static std::atomic<int> g_team_blocks{32};
+// SMs given to four-warp teams for the longest orbits (gal_set_team), or -1: as
+// many as the first pass's step counts suggest; atomic because calls on other
+// threads may read it while it is set
+static std::atomic<int> g_team_blocks{-1};
 // Fraction of every span the first pass of the two-pass schedule covers
 // (gal_set_split_fraction), in millionths
 static std::atomic<int> g_split_ppm{100000};
-
-// One library-owned stream per device for the team kernel, created on first use.
-static cudaError_t team_stream(cudaStream_t* out) {
-  static std::mutex mu;
-  static cudaStream_t streams[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!streams[dev]) {
-    e = cudaStreamCreateWithFlags(&streams[dev], cudaStreamNonBlocking);
-    if (e != cudaSuccess) return e;
-  }
-  *out = streams[dev];
-  return cudaSuccess;
-}
-
-// The fork/join event pair that orders the team stream after, and the caller's
-// stream before, one team launch. Created once per thread and device and then
-// reused: an event is re-recorded by every call, and cudaStreamWaitEvent takes
-// the record current at the time of the wait, so a pair must not be shared
-// between threads that launch concurrently.
-struct TeamEvents {
-  cudaEvent_t ev[64][2] = {};
-  ~TeamEvents() {
-    for (auto& p : ev)
-      for (cudaEvent_t e : p)
-        if (e) cudaEventDestroy(e);
-  }
-};
-
-static cudaError_t team_events(cudaEvent_t* fork, cudaEvent_t* join) {
-  thread_local TeamEvents cache;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  for (int k = 0; k < 2; ++k) {
-    if (!cache.ev[dev][k]) {
-      e = cudaEventCreateWithFlags(&cache.ev[dev][k], cudaEventDisableTiming);
-      if (e != cudaSuccess) {
-        cache.ev[dev][k] = nullptr;
-        return e;
-      }
-    }
-  }
-  *fork = cache.ev[dev][0];
-  *join = cache.ev[dev][1];
-  return cudaSuccess;
-}
 
 // Launch shape per [method == 8][adaptive], set by gal_set_launch. Dopri5 fits
 // 3 blocks of 128 per SM without spills (variant 0); Dopri8 needs the uncapped
@@ -267,7 +217,15 @@ gal_status validate_cfg(const gal_solver_config* c) {
 }
 
 // ---- two-phase schedule: order parked orbits by estimated remaining work
-constexpr int kBuckets = 64;
+constexpr int kBuckets = 120;  // sixths of an octave of remaining step attempts
+// The first pass ends an orbit's part after this many step attempts at the
+// latest: the longest orbits' rates are known by then, and a tenth of their spans
+// would be thousands of steps, in which most lanes have nothing left to do
+// (65,536 uneven orbits, s: 0.59 at 512, 0.59-0.70 at 256, 0.60 at 1024, 0.65
+// without this bound).
+constexpr int kParkSteps = 512;
+// Lone-thread to team time per step attempt.
+constexpr float kTeamRatio5 = 2.7f, kTeamRatio8 = 3.5f;
 
 __global__ void k_sched_keys(const OrbitResume* __restrict__ r, int64_t n, unsigned* __restrict__ hist,
                              int* __restrict__ bucket) {
@@ -275,7 +233,7 @@ __global__ void k_sched_keys(const OrbitResume* __restrict__ r, int64_t n, unsig
     if (r[i].paused) {
       const double p = r[i].progress;
       const double key = (double)r[i].nsteps * (1.0 - p) / fmax(p, 1e-12);
-      int b = (int)(2.0f * log2f(1.0f + (float)key));  // half-octave buckets
+      int b = (int)(6.0f * log2f(1.0f + (float)key));
       b = b < 0 ? 0 : (b >= kBuckets ? kBuckets - 1 : b);
       bucket[i] = b;
       atomicAdd(&hist[b], 1u);
@@ -285,16 +243,64 @@ __global__ void k_sched_keys(const OrbitResume* __restrict__ r, int64_t n, unsig
   }
 }
 
+// Step attempts of an orbit in bucket b: its lower edge times 2^(part / 6).
+__device__ __forceinline__ float bucket_work(int b, float part) { return exp2f(((float)b + part) / 6.0f) - 1.0f; }
+
+// Bucket cursors, most remaining work first, and the number of SMs that get a
+// team (one warp).
+//
+// A team's attempt takes 1 / ratio of a lone thread's, but an SM runs 16 orbits
+// on a team and 128 without. With t teams taking the 16 t longest orbits, the
+// batch ends no earlier than its longest orbit on a team, the longest other one
+// on a thread, and the whole work at the SMs' joint rate; t is the smallest
+// number that minimises the latest of the three. Measured (Dopri5, s): 65,536
+// uneven orbits 0.77 with 48 SMs, 0.59 with 64, 0.60 with 80 and 96, and 0.57 with
+// this choice; 262,144 of them 1.19 with 32, 1.22 with 64, 1.50 with 96, and 1.14.
 __global__ void k_sched_scan(const unsigned* __restrict__ hist, unsigned* __restrict__ cursor,
-                             unsigned long long* __restrict__ qlen) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
+                             unsigned long long* __restrict__ qlen, unsigned* __restrict__ teams, int sms,
+                             int fixed_teams, float ratio) {
+  const int lane = threadIdx.x;
+  if (lane == 0) {
     unsigned acc = 0;
-    for (int b = kBuckets - 1; b >= 0; --b) {  // most remaining work first
+    for (int b = kBuckets - 1; b >= 0; --b) {
       cursor[b] = acc;
       acc += hist[b];
     }
     *qlen = acc;
   }
+  if (fixed_teams >= 0) {
+    if (lane == 0) *teams = (unsigned)fixed_teams;
+    return;
+  }
+  float total = 0.f, longest = 0.f;
+  for (int b = 0; b < kBuckets; ++b) {
+    const float w = bucket_work(b, 0.5f);
+    total += (float)hist[b] * w;
+    if (hist[b]) longest = w;
+  }
+  float best = 3.4e38f;
+  int best_t = 0;
+  for (int t = lane; t < sms; t += 32) {
+    unsigned left = 16u * (unsigned)t;  // orbits the teams take
+    int b = kBuckets - 1;
+    while (b > 0 && left >= hist[b]) left -= hist[b--];  // b: bucket of the longest one on a thread
+    const float tail = bucket_work(b, 1.0f) * ratio;
+    const float rate = (float)(sms - t) * (128.f / ratio) + (float)t * 16.f;
+    const float end = fmaxf(fmaxf(t > 0 ? longest : longest * ratio, tail), total / rate);
+    if (end < best) {
+      best = end;
+      best_t = t;
+    }
+  }
+  for (int m = 16; m >= 1; m >>= 1) {
+    const float e = __shfl_xor_sync(0xffffffffu, best, m);
+    const int t = __shfl_xor_sync(0xffffffffu, best_t, m);
+    if (e < best || (e == best && t < best_t)) {
+      best = e;
+      best_t = t;
+    }
+  }
+  if (lane == 0) *teams = (unsigned)best_t;
 }
 
 __global__ void k_sched_scatter(const int* __restrict__ bucket, int64_t n, unsigned* __restrict__ cursor,
@@ -305,6 +311,9 @@ __global__ void k_sched_scatter(const int* __restrict__ bucket, int64_t n, unsig
   }
 }
 
+constexpr size_t kSchedHeader = 1024;
+static_assert(16 + 8 * kBuckets + 4 <= kSchedHeader, "schedule header");
+
 struct SchedLayout {
   size_t header, resume, bucket, order, total;
 };
@@ -313,8 +322,8 @@ static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 static SchedLayout sched_layout(int64_t n) {
   SchedLayout L{};
-  L.header = 0;  // [0] queue counter, [8] queue length, [16] hist[64], [272] cursor[64]
-  L.resume = 1024;
+  L.header = 0;  // queue counter, queue length, hist[kBuckets], cursor[kBuckets], teams
+  L.resume = kSchedHeader;
   L.bucket = L.resume + align256(sizeof(OrbitResume) * (size_t)n);
   L.order = L.bucket + align256(sizeof(int) * (size_t)n);
   L.total = L.order + align256(sizeof(int32_t) * (size_t)n);
@@ -667,14 +676,13 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   // Dopri8 1.93 / 6.14 at 2,432 orbits, 2.50 / 6.12 at 4,864, 4.76 / 6.13 at
   // 9,728, 6.99 / 6.13 at 12,160; Dopri5 1.00 / 2.71, 1.26 / 2.71, 2.28 / 2.73,
   // 3.28 / 2.73.
-  if (p->is_mw && team_blocks > 0 && n <= (int64_t)kTeamOrbitsPerSm * sms) {
+  if (p->is_mw && team_blocks != 0 && n <= (int64_t)kTeamOrbitsPerSm * sms) {
     cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return cuda_fail(e, "clearing the work queue");
     int64_t blocks = (n + kTeamLanes - 1) / kTeamLanes;
     if (blocks > 2 * sms) blocks = 2 * sms;
-    const long long base = kTeamLanes * blocks;
-    e = cfg->method == 8 ? launch_integrate_team8(a, p->mw, base, (int)blocks, 0, s)
-                         : launch_integrate_team(a, p->mw, base, (int)blocks, 0, s);
+    e = cfg->method == 8 ? launch_integrate_team8(a, p->mw, (int)blocks, s)
+                         : launch_integrate_team(a, p->mw, (int)blocks, s);
     return finish(e, "integrate kernel launch (teams)");
   }
   if (!cfg->schedule) {
@@ -682,24 +690,27 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
     if (e != cudaSuccess) return cuda_fail(e, "clearing the work queue");
     return finish(launch(), "integrate kernel launch");
   }
-  // two phases: a fraction of every span (a tenth by default), then longest remaining work first
+  // two phases: a part of every span (at most a tenth by default), then longest remaining work first
   const SchedLayout L = sched_layout(n);
   auto* qlen = reinterpret_cast<unsigned long long*>(ws + 8);
   auto* hist = reinterpret_cast<unsigned*>(ws + 16);
   auto* cursor = reinterpret_cast<unsigned*>(ws + 16 + 4 * kBuckets);
+  auto* teams = reinterpret_cast<unsigned*>(ws + 16 + 8 * kBuckets);
   auto* resume = reinterpret_cast<OrbitResume*>(ws + L.resume);
   auto* bucket = reinterpret_cast<int*>(ws + L.bucket);
   auto* order2 = reinterpret_cast<int32_t*>(ws + L.order);
   cudaError_t e = cudaMemsetAsync(ws, 0, L.resume + sizeof(OrbitResume) * (size_t)n, s);
   if (e != cudaSuccess) return cuda_fail(e, "clearing the schedule scratch");
   a.split_frac = 1e-6 * g_split_ppm.load(std::memory_order_relaxed);
+  a.park_steps = kParkSteps;
   a.resume = resume;
   e = launch();
   if (e != cudaSuccess) return cuda_fail(e, "integrate kernel launch (first pass)");
   unsigned grid;
   grid_for(n, 256, &grid);
   k_sched_keys<<<grid, 256, 0, s>>>(resume, n, hist, bucket);
-  k_sched_scan<<<1, 32, 0, s>>>(hist, cursor, qlen);
+  k_sched_scan<<<1, 32, 0, s>>>(hist, cursor, qlen, teams, sms, team_blocks < sms - 1 ? team_blocks : sms - 1,
+                                cfg->method == 8 ? kTeamRatio8 : kTeamRatio5);
   k_sched_scatter<<<grid, 256, 0, s>>>(bucket, n, cursor, order2);
   e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -707,48 +718,9 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   a.phase = 1;
   a.order = order2;
   a.queue_len = qlen;
-  const int blocks = team_blocks < sms - 1 ? team_blocks : sms - 1;
-  if (blocks > 0 && p->is_mw) {
-    // The longest orbits go to four-warp teams on `blocks` SMs of their own
-    // (second stream), the rest to the one-thread kernel on the other SMs, one
-    // block per SM; results are the same either way.
-    const long long tcap = (long long)kTeamLanes * blocks;
-    const long long base = tcap + 128LL * (sms - blocks);
-    cudaStream_t ts = nullptr;
-    e = team_stream(&ts);
-    cudaEvent_t fork = nullptr, join = nullptr;
-    if (e == cudaSuccess) e = team_events(&fork, &join);
-    if (e == cudaSuccess) e = cudaEventRecord(fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(ts, fork, 0);
-    bool team_launched = false, joinable = false;
-    if (e == cudaSuccess) {
-      e = cfg->method == 8 ? launch_integrate_team8(a, p->mw, base, blocks, kExclusiveSmem, ts)
-                           : launch_integrate_team(a, p->mw, base, blocks, kExclusiveSmem, ts);
-      team_launched = e == cudaSuccess;
-    }
-    if (e == cudaSuccess) {
-      e = cudaEventRecord(join, ts);
-      joinable = e == cudaSuccess;
-    }
-    if (e == cudaSuccess) {
-      a.queue_base = tcap;
-      // one warp per sub-partition: two (256 threads) made the step 1.4x longer
-      e = cfg->method == 8
-              ? launch_integrate_dopri8_exclusive(a, p->mw, shape.variant, 128, sms - blocks, kExclusiveSmem, s)
-              : launch_integrate_dopri5_exclusive(a, p->mw, shape.variant, 128, sms - blocks, kExclusiveSmem, s);
-    }
-    // Whatever failed after the team kernel was queued, the caller's stream
-    // still waits for it, so the caller never frees buffers it is using.
-    if (joinable) {
-      const cudaError_t ej = cudaStreamWaitEvent(s, join, 0);
-      if (e == cudaSuccess) e = ej;
-    } else if (team_launched) {
-      // Under stream capture nothing has run yet and a synchronize would
-      // invalidate the caller's capture; the caller discards it on this error.
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap == cudaStreamCaptureStatusNone)
-        cudaStreamSynchronize(ts);
-    }
+  if (p->is_mw && team_blocks != 0 && sms > 1) {
+    e = cfg->method == 8 ? launch_integrate_mixed8(a, p->mw, teams, sms, s)
+                         : launch_integrate_mixed(a, p->mw, teams, sms, s);
     return finish(e, "integrate kernel launch (second pass, teams)");
   }
   return finish(launch(), "integrate kernel launch (second pass)");

@@ -111,11 +111,11 @@ struct IntegrateArgs {
   int64_t n;
   unsigned long long* queue;  // work-queue counter (scratch)
   const DevLinear* lin;       // time-dependent component parameters (table kernel), or NULL
-  long long queue_base;       // first queue position of this launch (earlier ones belong to a team kernel)
   // two-phase schedule: phase 0 parks every orbit once it has covered split_frac
   // of its span; phase 1 resumes the parked orbits from `resume` in `order`
   int32_t phase;
   double split_frac;                     // <= 0: single pass
+  int64_t park_steps;                    // ... or after this many step attempts
   OrbitResume* resume;                   // [n]
   double* defer;                         // Dopri8: start time of each deferred save's step [out_stride], or NULL
   const unsigned long long* queue_len;   // phase 1: number of entries in order (device)
@@ -418,11 +418,21 @@ __device__ __forceinline__ void first_step(const IntegrateArgs& a, OrbitState& s
 // With LANES = 32 a whole warp owns one orbit (warp-per-orbit mode, for
 // composites with many components): the positions are handed out per warp,
 // and lane 0 takes the next one from the queue for the warp.
+//
+// Blocks: the `count` blocks of a launch that share one arrangement, of which
+// this is number `index`, and their first queue position (all blocks and 0, but
+// in the mixed kernel of integrate_team.cuh).
+struct Blocks {
+  unsigned count, index;
+  long long base;
+};
+__device__ __forceinline__ Blocks all_blocks() { return Blocks{gridDim.x, blockIdx.x, 0}; }
+
 template <int LANES>
-__device__ __forceinline__ unsigned long long first_position() {
+__device__ __forceinline__ unsigned long long first_position(const Blocks& g) {
   const unsigned long long W = blockDim.x >> 5, w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if constexpr (LANES == 32) return w * gridDim.x + blockIdx.x;
-  return (l * W + w) * gridDim.x + blockIdx.x;
+  if constexpr (LANES == 32) return w * g.count + g.index;
+  return (l * W + w) * g.count + g.index;
 }
 
 template <int LANES>
@@ -437,16 +447,16 @@ __device__ __forceinline__ unsigned long long next_position(unsigned long long* 
 
 // Returns false when the queue is empty.
 template <class TB, class Pot, int LANES = 1>
-__device__ __forceinline__ bool start_orbit(const IntegrateArgs& a, const Pot& pot, OrbitState& s,
+__device__ __forceinline__ bool start_orbit(const IntegrateArgs& a, const Pot& pot, const Blocks& g, OrbitState& s,
                                             bool& first) {
   const unsigned long long qlen = a.queue_len ? *a.queue_len : (unsigned long long)a.n;
-  const unsigned long long striped = (unsigned long long)gridDim.x * (blockDim.x / LANES);
-  const unsigned long long base = (unsigned long long)a.queue_base;
+  const unsigned long long striped = (unsigned long long)g.count * (blockDim.x / LANES);
+  const unsigned long long base = (unsigned long long)g.base;
   while (true) {
     unsigned long long k;
     if (first) {
       first = false;
-      k = base + first_position<LANES>();
+      k = base + first_position<LANES>(g);
     } else {
       k = base + striped + next_position<LANES>(a.queue);
     }
@@ -483,7 +493,7 @@ __device__ __forceinline__ bool maybe_park(const IntegrateArgs& a, OrbitState& s
   if (a.phase != 0 || !gt_zero(a.split_frac)) return false;
   const double span = s.tau1 - s.tau0;
   const double done = s.tau - s.tau0;
-  if (lt_bits(done, a.split_frac * span)) return false;
+  if (s.nsteps < a.park_steps && lt_bits(done, a.split_frac * span)) return false;
   OrbitResume& r = a.resume[s.orbit];
 #pragma unroll
   for (int j = 0; j < 6; ++j) r.y[j] = s.y[j];
@@ -609,11 +619,11 @@ __device__ __forceinline__ double clip_to_end(double tprev, double tnext, double
 // the 32 lanes run the orbit's steps in lockstep on identical values and their
 // identical stores of saves, status and steps coincide.
 template <class TB, class Pot, int LANES = 1>
-__device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
+__device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot, const Blocks& g = all_blocks()) {
   OrbitState s;
   s.orbit = -1;
   bool first = true;
-  if (!start_orbit<TB, Pot, LANES>(a, pot, s, first)) return;
+  if (!start_orbit<TB, Pot, LANES>(a, pot, g, s, first)) return;
   double F[TB::S][6];
   while (true) {
     // One RK evaluation per iteration: either the main step from (tau, y) or,
@@ -646,7 +656,7 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
       else if (le_bits(s.tau1, s.tau)) done = true;
       else if (s.nsteps >= a.max_steps) { done = true; st = ORBIT_MAX_STEPS; }
       else if (maybe_park(a, s)) {
-        if (!start_orbit<TB, Pot, LANES>(a, pot, s, first)) return;
+        if (!start_orbit<TB, Pot, LANES>(a, pot, g, s, first)) return;
         continue;
       }
     } else {
@@ -721,14 +731,14 @@ __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot) {
         else if (le_bits(s.tau1, s.tau)) done = true;
         else if (s.nsteps >= a.max_steps) { done = true; st = ORBIT_MAX_STEPS; }
         else if (maybe_park(a, s)) {
-          if (!start_orbit<TB, Pot, LANES>(a, pot, s, first)) return;
+          if (!start_orbit<TB, Pot, LANES>(a, pot, g, s, first)) return;
           continue;
         }
       }
     }
     if (done) {
       finish_orbit(a, s, st);
-      if (!start_orbit<TB, Pot, LANES>(a, pot, s, first)) return;
+      if (!start_orbit<TB, Pot, LANES>(a, pot, g, s, first)) return;
     }
   }
 }

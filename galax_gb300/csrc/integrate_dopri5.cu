@@ -1,5 +1,6 @@
 // Dopri5 instantiation of the orbit-integration kernels, and the four-warp
-// team kernel for the longest orbits of a two-pass Milky Way batch.
+// team kernels for small batches and for the longest orbits of a two-pass batch
+// in the Milky Way model.
 #include "integrate_kernels.cuh"
 #include "integrate_team.cuh"
 
@@ -9,20 +10,17 @@ cudaError_t launch_integrate_dopri5(const IntegrateArgs& a, bool mw, const MWPar
   return launch_integrate<Dopri5>(a, mw, p, comps, ncomp, shape, stream);
 }
 
-cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, long long base, int blocks, size_t smem,
-                                  cudaStream_t stream) {
-  if (smem > 0) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_integrate_mw_team<Dopri5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  k_integrate_mw_team<Dopri5><<<(unsigned)blocks, 128, smem, stream>>>(a, p, base);
+cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream) {
+  k_integrate_mw_team<Dopri5><<<(unsigned)blocks, 128, 0, stream>>>(a, p);
   return cudaGetLastError();
 }
 
-cudaError_t launch_integrate_dopri5_exclusive(const IntegrateArgs& a, const MWParams& p, int variant, int block,
-                                              int grid, size_t smem, cudaStream_t stream) {
-  if (variant != 2 && block > 128) block = 128;  // variants 0 and 1 are built for at most 128 threads
-  return mw_launch_exclusive<Dopri5>(variant, (unsigned)grid, block, smem, stream, a, p);
+cudaError_t launch_integrate_mixed(const IntegrateArgs& a, const MWParams& p, const unsigned* teams, int blocks,
+                                   cudaStream_t stream) {
+  const cudaError_t e = cudaFuncSetAttribute(k_integrate_mw_mixed<Dopri5>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kExclusiveSmem);
+  if (e != cudaSuccess) return e;
+  k_integrate_mw_mixed<Dopri5><<<(unsigned)blocks, 128, kExclusiveSmem, stream>>>(a, p, teams);
+  return cudaGetLastError();
 }
 }  // namespace gal

@@ -155,11 +155,10 @@ __device__ __forceinline__ void team_write_save(const IntegrateArgs& a, const Or
   a.out[j * a.out_stride + save_index(a, s, k)] = v;
 }
 
-// Takes queue positions [0, 16 gridDim.x) in stripes, then base +
-// atomicAdd(queue) (base: the positions that this launch and one running beside
-// it on the same queue hand out in stripes).
+// Takes queue positions [0, 16 g.count) in stripes, then base + atomicAdd(queue)
+// (base: all positions that this launch hands out in stripes).
 template <class TB>
-__global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, MWParams p, long long base) {
+__device__ void team_loop(const IntegrateArgs& a, const MWParams& p, const Blocks& g, long long base) {
   constexpr int S = TB::S;
   constexpr double kIdle = 8.0;  // position of lanes without an orbit
   __shared__ TeamShared sh;
@@ -179,7 +178,7 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
   while (true) {
     // ---- orbits for free lanes (warp 0 dequeues)
     if (warp == 0 && !hi && need_orbit && queue_open) {
-      const long long k = first ? (long long)slot * gridDim.x + blockIdx.x : base + (long long)atomicAdd(a.queue, 1ULL);
+      const long long k = first ? (long long)slot * g.count + g.index : base + (long long)atomicAdd(a.queue, 1ULL);
       sh.slot[slot] = k < qlen ? (a.order ? (long long)a.order[k] : k) : -1;
     }
     first = false;
@@ -225,8 +224,8 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
     // round, only when a lane needs it
     const bool want_f0 = fresh || (need_f0 && active);
     if (__syncthreads_or(want_f0)) {
-      const double g = team_grad(sh, warp, lane, p, want_f0 ? yp : kIdle);
-      if (want_f0) F0v = -g;
+      const double gr = team_grad(sh, warp, lane, p, want_f0 ? yp : kIdle);
+      if (want_f0) F0v = -gr;
     }
     need_f0 = false;
     // ---- first step of orbits that start here (start_orbit, initial_step)
@@ -244,10 +243,10 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
 #pragma unroll
       for (int j = 0; j < 6; ++j) F0[j] = sh.y1[j][slot];
       if (probe) is = initial_probe(a, s.y, F0);
-      const double g = team_grad(sh, warp, lane, p, probe ? fma(is.h0 * s.dir, yv, yp) : kIdle);
+      const double gr = team_grad(sh, warp, lane, p, probe ? fma(is.h0 * s.dir, yv, yp) : kIdle);
       if (owner && !hi) {
         sh.err[j0][slot] = fma(is.h0 * s.dir, F0v, yv);
-        sh.err[j1][slot] = -g;
+        sh.err[j1][slot] = -gr;
       }
       __syncthreads();
       if (probe) {
@@ -410,6 +409,26 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
       need_orbit = true;
       need_f0 = false;
     }
+  }
+}
+
+// A whole batch on teams, two blocks per SM.
+template <class TB>
+__global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, MWParams p) {
+  team_loop<TB>(a, p, all_blocks(), (long long)kTeamLanes * gridDim.x);
+}
+
+// Second pass of the two-pass schedule, one block of 128 threads per SM: the
+// first *teams blocks are teams and take the longest orbits, the others run one
+// thread per orbit; when their first orbits are done, all draw on one queue.
+template <class TB>
+__global__ void __launch_bounds__(128, 1) k_integrate_mw_mixed(IntegrateArgs a, MWParams p, const unsigned* teams) {
+  const unsigned t = min(*teams, gridDim.x - 1);
+  const long long first = (long long)kTeamLanes * t;  // queue position of the longest orbit without a team
+  if (blockIdx.x < t) {
+    team_loop<TB>(a, p, Blocks{t, blockIdx.x, 0}, first + 128LL * (gridDim.x - t));
+  } else {
+    integrate_loop<TB>(a, MWPot{p}, Blocks{gridDim.x - t, blockIdx.x - t, first});
   }
 }
 

@@ -22,22 +22,17 @@ cudaError_t launch_integrate_dopri5(const IntegrateArgs& a, bool mw, const MWPar
 cudaError_t launch_integrate_dopri8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps,
                                     int ncomp, LaunchShape shape, cudaStream_t stream);
 
-// Four-warp teams (16 orbits per block) for a Milky Way Dopri5 batch: queue
-// positions [0, 16 blocks) in stripes, then base + atomicAdd(a.queue). smem:
-// dynamic shared memory requested (unused) to keep other kernels off the
-// blocks' SMs.
-cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, long long base, int blocks, size_t smem,
-                                  cudaStream_t stream);
-// The one-thread Milky Way Dopri5 kernel, `block` threads per block, `grid`
-// blocks, each requesting `smem` bytes (unused) so that blocks of this launch
-// and of the team launch never share an SM.
-cudaError_t launch_integrate_dopri5_exclusive(const IntegrateArgs& a, const MWParams& p, int variant, int block,
-                                              int grid, size_t smem, cudaStream_t stream);
-// The same two launches for a Dopri8 batch.
-cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, long long base, int blocks, size_t smem,
+// A Milky Way batch on `blocks` four-warp teams (16 orbits per block).
+cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream);
+cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream);
+// The second pass of such a batch on `blocks` SMs, *teams (device memory) of them
+// with a team and the others with one thread per orbit. Every block requests
+// kExclusiveSmem bytes of dynamic shared memory, which it does not use, so that
+// no two share an SM.
+cudaError_t launch_integrate_mixed(const IntegrateArgs& a, const MWParams& p, const unsigned* teams, int blocks,
                                    cudaStream_t stream);
-cudaError_t launch_integrate_dopri8_exclusive(const IntegrateArgs& a, const MWParams& p, int variant, int block,
-                                              int grid, size_t smem, cudaStream_t stream);
+cudaError_t launch_integrate_mixed8(const IntegrateArgs& a, const MWParams& p, const unsigned* teams, int blocks,
+                                    cudaStream_t stream);
 // Dopri8 saves left to a.defer (put_deferred_save), after the integration on the same stream.
 cudaError_t launch_deferred_saves8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
                                    cudaStream_t stream);

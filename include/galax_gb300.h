@@ -152,7 +152,8 @@ typedef struct gal_solver_config {
   double safety, factormin, factormax;
   int32_t force_dtmin;
   /* 0: one pass. 1: two passes over the batch with identical results: every
-   * orbit first covers the first tenth of its time span, then the orbits are
+   * orbit first covers the first tenth of its time span (or 512 step attempts,
+   * if those come first), then the orbits are
    * resumed in order of decreasing estimated remaining work (steps so far x
    * remaining fraction), so the longest orbits start early instead of forming a
    * tail. Useful for adaptive batches with uneven lengths. */
@@ -258,13 +259,14 @@ GAL_API gal_status gal_dense_evaluate(const gal_potential* pot, int32_t method, 
 GAL_API gal_status gal_set_launch(int32_t method, int32_t adaptive, int32_t block_threads, int32_t blocks_per_sm,
                                   int32_t variant);
 /* Four-warp team blocks (16 orbits each, two Runge-Kutta stages per round) in
- * the Milky Way model. blocks > 0 (default 32, at most the SM count - 1): small
- * batches run on teams alone, and the second pass of a larger two-pass batch
- * gives `blocks` SMs to teams, which take the longest orbits first, on a
- * library-owned stream beside the one-thread-per-orbit kernel, which runs one
- * block per remaining SM. 0 keeps every orbit on the one-thread kernel with the
- * launch shape of gal_set_launch. Results are bitwise identical either way; the
- * teams cut the serial latency of few or long orbits. Process-wide. */
+ * the Milky Way model. blocks > 0 (at most the SM count - 1): small batches run
+ * on teams alone, and the second pass of a larger two-pass batch gives `blocks`
+ * SMs to teams, which take the longest orbits first, while the other SMs run one
+ * thread per orbit; until it is set, that number is chosen for each batch on the
+ * device from the first pass's step counts. 0 keeps every orbit on the one-thread
+ * kernel with the launch shape of gal_set_launch. Results are bitwise identical
+ * either way; the teams cut the serial latency of few or long orbits.
+ * Process-wide. */
 GAL_API gal_status gal_set_team(int32_t blocks);
 /* Fraction of every orbit's span that the first pass of the two-pass schedule
  * (cfg->schedule = 1) covers before the orbits are ordered by their remaining
