@@ -67,6 +67,8 @@ class StreamConfig(C.Structure):
     ]
 
 
+GAL_EVAL_POTENTIAL, GAL_EVAL_GRADIENT, GAL_EVAL_ACCELERATION, GAL_EVAL_HESSIAN = range(4)
+
 STREAM_DF_OFFSETS = 0
 STREAM_DF_FARDAL2015 = 1
 STREAM_DF_CHEN2024 = 2
@@ -89,6 +91,8 @@ SIGNATURES = {
     "gal_eval_gradient": (C.c_int, [C.c_void_p, _DP, C.c_double, C.c_int64, _DP, C.c_void_p]),
     "gal_eval_acceleration": (C.c_int, [C.c_void_p, _DP, C.c_double, C.c_int64, _DP, C.c_void_p]),
     "gal_eval_hessian": (C.c_int, [C.c_void_p, _DP, C.c_double, C.c_int64, _DP, C.c_void_p]),
+    "gal_eval_points": (C.c_int, [C.c_void_p, C.c_int32, _DP, C.c_int64, C.c_int64, C.c_double, C.c_int64, _DP,
+                                  C.c_void_p]),
     "gal_integrate_workspace_size": (C.c_int, [C.POINTER(SolverConfig), C.c_int64, C.POINTER(C.c_size_t)]),
     "gal_integrate_workspace_size_saves": (C.c_int, [C.POINTER(SolverConfig), C.c_int64, C.c_int64,
                                                      C.POINTER(C.c_size_t)]),

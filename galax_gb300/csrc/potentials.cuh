@@ -567,4 +567,41 @@ struct MWPot {
   }
 };
 
+// The Hessian of the same four components: H = {xx, xy, xz, yy, yz, zz}. For a
+// sphere grad Phi = g x and H = g 1 + (g'/r) x x^T; with d = r + c,
+//   Hernquist  g = G m / (r d^2),              g'/r = -g (1/r^2 + 2 / (r d)),
+//   NFW        g = G m (L/r - 1/d) / r^2,      g'/r = (G m / d^2 / r - 3 g) / r^2.
+__device__ __forceinline__ void mw_hessian(const MWParams& p, double x, double y, double z, double* H) {
+  double r;
+  const double ir = mw_ir(x, y, z, r);
+  const double ir2 = ir * ir;
+  const double dh = p.rs_h + r, db = r + p.rs_b, dn = r + p.rs_n;
+  const double bn = db * dn;
+  const double iP = 1.0 / (dh * bn);
+  const double idh = iP * bn, ih = iP * dh, idb = ih * dn, idn = ih * db;
+  const double L = mw_halo_log(p, r);
+  const double gh = p.Gm_h * ir2 * fma(L, ir, -idh);
+  const double gb = p.Gm_b * ir * (idb * idb), gn = p.Gm_n * ir * (idn * idn);
+  const double gpr = ir2 * fma(p.Gm_h * ir, idh * idh, -3.0 * gh) -
+                     fma(gb, fma(2.0 * ir, idb, ir2), gn * fma(2.0 * ir, idn, ir2));
+  const double g = gh + (gb + gn);
+  // disk: u = G m / D^3, w = 3 G m / D^5, v = (x, y, z s / zb)
+  const double zb2 = fma(z, z, p.b2_d);
+  const double izb = rsqrt(zb2);
+  const double s = fma(zb2, izb, p.a_d);
+  const double iD = rsqrt(fma(s, s, fma(x, x, y * y)));
+  const double iD2 = iD * iD;
+  const double u = p.Gm_d * iD2 * iD;
+  const double w = 3.0 * u * iD2;
+  const double vz = z * (s * izb);
+  const double d = u + g;
+  const double px = (gpr - w) * x, py = (gpr - w) * y;
+  H[0] = fma(px, x, d);
+  H[1] = px * y;
+  H[2] = x * fma(gpr, z, -w * vz);
+  H[3] = fma(py, y, d);
+  H[4] = y * fma(gpr, z, -w * vz);
+  H[5] = fma(gpr * z, z, fma(-w * vz, vz, fma(u * (p.a_d * p.b2_d), izb * izb * izb, d)));
+}
+
 }  // namespace gal

@@ -117,14 +117,14 @@ class AbstractPotential:
     def handle(self) -> int:
         """The device-side ``gal_potential`` for the current CUDA device."""
         torch = _torch()
+        recs, slopes = self.components(), self.slopes()
+        key = (recs, self.G, None if slopes is None else slopes.tobytes())
+        if self._handle is not None and self._handle_key == key and self._handle_device == torch.cuda.current_device():
+            return self._handle
         if not torch.cuda.is_available():
             raise _lib.GalaxGB300Error("no CUDA device: the galax_gb300 path has no CPU fallback")
         dev = torch.cuda.current_device()
         arr = self.component_array()
-        slopes = self.slopes()
-        key = arr.tobytes() + np.float64(self.G).tobytes() + (b"" if slopes is None else slopes.tobytes())
-        if self._handle is not None and self._handle_device == dev and self._handle_key == key:
-            return self._handle
         self._release()
         L = _lib.load()
         h = C.c_void_p()
@@ -155,44 +155,45 @@ class AbstractPotential:
         return bool(_lib.load().gal_potential_is_milky_way(self.handle()))
 
     # ---- evaluation --------------------------------------------------------
-    def _positions(self, x):
+    @staticmethod
+    def _positions(x):
+        """(n, 3) float64 CUDA view (or copy, if it was not that) of x, its batch shape, whether x was NumPy's."""
         torch = _torch()
         is_np = not isinstance(x, torch.Tensor)
         xt = torch.as_tensor(np.asarray(x, dtype=np.float64) if is_np else x)
         if xt.shape[-1] != 3:
             raise ValueError(f"positions must have a last axis of size 3, got shape {tuple(xt.shape)}")
-        batch = xt.shape[:-1]
-        soa = xt.reshape(-1, 3).to(device="cuda", dtype=torch.float64).t().contiguous()
-        return soa, batch, is_np
+        return xt.reshape(-1, 3).to(device="cuda", dtype=torch.float64), xt.shape[:-1], is_np
 
     @staticmethod
     def _out(t, is_np):
         return t.cpu().numpy() if is_np else t
 
-    def _eval(self, fn: str, x, t, ncomp_out: int):
+    def _eval(self, what: int, x, t, ncomp_out: int):
         torch = _torch()
-        soa, batch, is_np = self._positions(x)
-        n = soa.shape[1]
+        pts, batch, is_np = self._positions(x)
+        n = pts.shape[0]
         out = torch.empty((ncomp_out, n), dtype=torch.float64, device="cuda")
-        L = _lib.load()
-        stream = torch.cuda.current_stream().cuda_stream
-        _lib.check(getattr(L, fn)(self.handle(), soa.data_ptr(), float(t or 0.0), n, out.data_ptr(), stream), fn)
+        h = self.handle()
+        st = _lib.load().gal_eval_points(h, what, pts.data_ptr(), pts.stride(0), pts.stride(1), float(t or 0.0), n,
+                                         out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        _lib.check(st, "gal_eval_points")
         return out, batch, is_np
 
     def potential(self, x, t=0.0):
-        out, batch, is_np = self._eval("gal_eval_potential", x, t, 1)
+        out, batch, is_np = self._eval(_lib.GAL_EVAL_POTENTIAL, x, t, 1)
         return self._out(out.reshape(batch), is_np)
 
     def gradient(self, x, t=0.0):
-        out, batch, is_np = self._eval("gal_eval_gradient", x, t, 3)
+        out, batch, is_np = self._eval(_lib.GAL_EVAL_GRADIENT, x, t, 3)
         return self._out(out.t().reshape(*batch, 3), is_np)
 
     def acceleration(self, x, t=0.0):
-        out, batch, is_np = self._eval("gal_eval_acceleration", x, t, 3)
+        out, batch, is_np = self._eval(_lib.GAL_EVAL_ACCELERATION, x, t, 3)
         return self._out(out.t().reshape(*batch, 3), is_np)
 
     def hessian(self, x, t=0.0):
-        out, batch, is_np = self._eval("gal_eval_hessian", x, t, 9)
+        out, batch, is_np = self._eval(_lib.GAL_EVAL_HESSIAN, x, t, 9)
         return self._out(out.t().reshape(*batch, 3, 3), is_np)
 
     def local_circular_velocity(self, x, t=0.0):

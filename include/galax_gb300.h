@@ -136,6 +136,12 @@ GAL_API gal_status gal_eval_acceleration(const gal_potential* pot, const double*
                                  gal_stream_t stream);
 GAL_API gal_status gal_eval_hessian(const gal_potential* pot, const double* x, double t, int64_t n, double* out,
                             gal_stream_t stream);
+/* The same for positions in any layout (component j of point i at
+ * x[i point_stride + j axis_stride], in doubles), so that a caller's array of
+ * points is read where it is. what: which of the four; out as above. */
+enum { GAL_EVAL_POTENTIAL = 0, GAL_EVAL_GRADIENT = 1, GAL_EVAL_ACCELERATION = 2, GAL_EVAL_HESSIAN = 3 };
+GAL_API gal_status gal_eval_points(const gal_potential* pot, int32_t what, const double* x, int64_t point_stride,
+                           int64_t axis_stride, double t, int64_t n, double* out, gal_stream_t stream);
 
 /* ------------------------------------------------------------------ integration */
 /* Solver configuration; field meanings follow diffrax's Dopri5/Dopri8,
