@@ -703,13 +703,14 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   // Dopri8 1.93 / 6.14 at 2,432 orbits, 2.50 / 6.12 at 4,864, 4.76 / 6.13 at
   // 9,728, 6.99 / 6.13 at 12,160; Dopri5 1.00 / 2.71, 1.26 / 2.71, 2.28 / 2.73,
   // 3.28 / 2.73.
-  if (p->is_mw && team_blocks != 0 && n <= (int64_t)kTeamOrbitsPerSm * sms) {
+  if (team_blocks != 0 && n <= (int64_t)kTeamOrbitsPerSm * sms &&
+      (p->is_mw || (p->n <= kTeamMaxComps && shape.table_lanes == 0))) {
     cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return cuda_fail(e, "clearing the work queue");
     int64_t blocks = (n + kTeamLanes - 1) / kTeamLanes;
     if (blocks > 2 * sms) blocks = 2 * sms;
-    e = cfg->method == 8 ? launch_integrate_team8(a, p->mw, (int)blocks, s)
-                         : launch_integrate_team(a, p->mw, (int)blocks, s);
+    e = cfg->method == 8 ? launch_integrate_team8(a, p->is_mw, p->mw, p->d_comps, p->n, (int)blocks, s)
+                         : launch_integrate_team(a, p->is_mw, p->mw, p->d_comps, p->n, (int)blocks, s);
     return finish(e, "integrate kernel launch (teams)");
   }
   if (!cfg->schedule) {

@@ -75,7 +75,8 @@ __device__ __forceinline__ double sixth(double a) {
   return fma(fma(-6.0, q, a), y, q);
 }
 
-constexpr int kTeamLanes = 16;  // orbits per four-warp team block (integrate_team.cuh)
+constexpr int kTeamLanes = 16;     // orbits per four-warp team block (integrate_team.cuh)
+constexpr int kTeamMaxComps = 16;  // components of a table that teams take
 
 // Everything needed to continue an orbit exactly where a first pass parked it
 // (state, step times, controller memory, counters, save cursor). 128 bytes.

@@ -10,8 +10,11 @@ cudaError_t launch_integrate_dopri5(const IntegrateArgs& a, bool mw, const MWPar
   return launch_integrate<Dopri5>(a, mw, p, comps, ncomp, shape, stream);
 }
 
-cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream) {
-  k_integrate_mw_team<Dopri5><<<(unsigned)blocks, 128, 0, stream>>>(a, p);
+cudaError_t launch_integrate_team(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                   int blocks, cudaStream_t stream) {
+  if (mw) k_integrate_mw_team<Dopri5><<<(unsigned)blocks, 128, 0, stream>>>(a, p);
+  else if (a.lin) k_integrate_table_team<Dopri5, true><<<(unsigned)blocks, 128, 0, stream>>>(a, comps, ncomp);
+  else k_integrate_table_team<Dopri5, false><<<(unsigned)blocks, 128, 0, stream>>>(a, comps, ncomp);
   return cudaGetLastError();
 }
 

@@ -19,8 +19,11 @@ bool dopri8_warp_per_orbit(const LaunchShape& shape, int64_t n, int ncomp) {
   return use_warp_per_orbit(shape, n, ncomp);
 }
 
-cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream) {
-  k_integrate_mw_team<Dopri8><<<(unsigned)blocks, 128, 0, stream>>>(a, p);
+cudaError_t launch_integrate_team8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                   int blocks, cudaStream_t stream) {
+  if (mw) k_integrate_mw_team<Dopri8><<<(unsigned)blocks, 128, 0, stream>>>(a, p);
+  else if (a.lin) k_integrate_table_team<Dopri8, true><<<(unsigned)blocks, 128, 0, stream>>>(a, comps, ncomp);
+  else k_integrate_table_team<Dopri8, false><<<(unsigned)blocks, 128, 0, stream>>>(a, comps, ncomp);
   return cudaGetLastError();
 }
 

@@ -1,5 +1,5 @@
 // Four-warp teams with paired stages: the latency-optimal arrangement for few
-// or long orbits in the Milky Way model.
+// or long orbits.
 //
 // A lone orbit is bound by its chain of FP64 instructions: a GB300 FP64 warp
 // instruction holds its sub-partition's FP64 pipe for 64 cycles (76 with all
@@ -15,7 +15,8 @@
 // one pass of the gradient code serves both. Dopri5 takes 3 rounds a step
 // instead of 6, Dopri8 6 (and one for the next step's first slope) instead of 13.
 //
-// Four warps per gradient:
+// Four warps per gradient. In the Milky Way model (a table's components are
+// shared out likewise):
 //   warp 0: the spheres' radius, the shared reciprocal, the bulge and nucleus;
 //   warp 1: the radius and the NFW halo's log(1 + r / r_s) (mw_halo_log);
 //   warp 2: the radius and the halo's factor;
@@ -45,8 +46,6 @@ namespace gal {
 struct TeamShared {
   // field-evaluation exchange: lane = 16 * (stage of the pair) + orbit
   double pos[3][32];
-  double u[32], us[32], izb[32];
-  double A[32], B[32], inv_dh[32], ir[32], L[32];
   // controller exchange
   double y1[6][kTeamLanes], err[6][kTeamLanes];
   long long slot[kTeamLanes];
@@ -118,37 +117,123 @@ __device__ __forceinline__ double dense_comp(double y0j, double hs, const double
   return fma(hs, acc, y0j);
 }
 
-// One round of field evaluations, a point per lane: the owners (warps 0-2) hold
-// their position component `q`; returns warp w's gradient component (w < 3).
-__device__ __forceinline__ double team_grad(TeamShared& sh, int warp, int lane, const MWParams& p, double q) {
-  if (warp < 3) sh.pos[warp][lane] = q;
-  __syncthreads();  // positions written
-  const double x = sh.pos[0][lane], y = sh.pos[1][lane], z = sh.pos[2][lane];
-  if (warp == 3) {
-    const MWDisk d = mw_disk(p, x, y, z);
-    sh.u[lane] = d.u;
-    sh.us[lane] = d.us;
-    sh.izb[lane] = d.izb;
-  } else {  // mw_f's products where their factors are
-    double r;
-    const double ir = mw_ir(x, y, z, r);
-    if (warp == 0) {
-      const MWRecip c = mw_recip(p, r);
-      sh.B[lane] = ir * fma(p.Gm_b, c.inv_db2, p.Gm_n * c.inv_dn2);
-      sh.inv_dh[lane] = c.inv_dh;
-    } else if (warp == 1) {
-      sh.L[lane] = mw_halo_log(p, r);
-    } else {
-      sh.A[lane] = p.Gm_h * (ir * ir);
-      sh.ir[lane] = ir;
+// Models: grad() is one round of field evaluations, a point per lane, at time t.
+// The owners (warps 0-2) hold their position component q; warp w < 3 gets its
+// gradient component.
+//
+// The Milky Way.
+struct TeamMW {
+  static constexpr bool TIMED = false;
+  struct Shared {
+    double u[32], us[32], izb[32];
+    double A[32], B[32], inv_dh[32], ir[32], L[32];
+  };
+  const MWParams& p;
+  Shared& m;
+
+  __device__ __forceinline__ double grad(TeamShared& sh, int warp, int lane, double q, double) const {
+    if (warp < 3) sh.pos[warp][lane] = q;
+    __syncthreads();  // positions written
+    const double x = sh.pos[0][lane], y = sh.pos[1][lane], z = sh.pos[2][lane];
+    if (warp == 3) {
+      const MWDisk d = mw_disk(p, x, y, z);
+      m.u[lane] = d.u;
+      m.us[lane] = d.us;
+      m.izb[lane] = d.izb;
+    } else {  // mw_f's products where their factors are
+      double r;
+      const double ir = mw_ir(x, y, z, r);
+      if (warp == 0) {
+        const MWRecip c = mw_recip(p, r);
+        m.B[lane] = ir * fma(p.Gm_b, c.inv_db2, p.Gm_n * c.inv_dn2);
+        m.inv_dh[lane] = c.inv_dh;
+      } else if (warp == 1) {
+        m.L[lane] = mw_halo_log(p, r);
+      } else {
+        m.A[lane] = p.Gm_h * (ir * ir);
+        m.ir[lane] = ir;
+      }
+    }
+    __syncthreads();  // pieces written
+    if (warp > 2) return 0.0;
+    const double f = m.A[lane] * fma(m.L[lane], m.ir[lane], -m.inv_dh[lane]) + m.B[lane];
+    if (warp < 2) return (m.u[lane] + f) * q;
+    return fma(m.us[lane], m.izb[lane], f) * q;
+  }
+};
+
+// A table of up to kTeamMaxComps components: each warp evaluates the factors of
+// its share (spread by their FP64 instruction counts), and the owners sum them in
+// the table's order, as TablePot does. 3,001 orbits in MilkyWayPotential2022
+// (default integrator, 1.5 Gyr, 77 saves): 79 ms on single threads, 26 on teams.
+template <bool TIMED_>
+struct TeamTable {
+  static constexpr bool TIMED = TIMED_;
+  struct Shared {
+    double fxy[kTeamMaxComps][32], fz[kTeamMaxComps][32];
+    DevComp c[kTeamMaxComps];
+    int warp[kTeamMaxComps];
+  };
+  int n;
+  const DevLinear* lin;
+  Shared& m;
+
+  // Components into shared memory, the costliest first to the warp with least.
+  __device__ __forceinline__ void stage(const DevComp* comps) const {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) m.c[i] = comps[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int load[4] = {0, 0, 0, 0};
+      for (int i = 0; i < n; ++i) m.warp[i] = -1;
+      for (int k = 0; k < n; ++k) {
+        int best = -1, cost = -1;
+        for (int i = 0; i < n; ++i)
+          if (m.warp[i] < 0 && team_cost(m.c[i].kind) > cost) cost = team_cost(m.c[best = i].kind);
+        int w = 3;
+        for (int v = 2; v >= 0; --v)
+          if (load[v] < load[w]) w = v;
+        m.warp[best] = w;
+        load[w] += cost;
+      }
+    }
+    __syncthreads();
+  }
+
+  static __device__ __forceinline__ int team_cost(int kind) {  // FP64 instructions of one gradient
+    switch (kind) {
+      case NFW: return 42;
+      case POWERLAW_CUTOFF: return 400;
+      case MIYAMOTO_NAGAI: return 22;
+      case HERNQUIST: return 22;
+      case ISOCHRONE: return 28;
+      default: return 16;
     }
   }
-  __syncthreads();  // pieces written
-  if (warp > 2) return 0.0;
-  const double f = sh.A[lane] * fma(sh.L[lane], sh.ir[lane], -sh.inv_dh[lane]) + sh.B[lane];
-  if (warp < 2) return (sh.u[lane] + f) * q;
-  return fma(sh.us[lane], sh.izb[lane], f) * q;
-}
+
+  __device__ __forceinline__ double grad(TeamShared& sh, int warp, int lane, double q, double t) const {
+    if (warp < 3) sh.pos[warp][lane] = q;
+    __syncthreads();  // positions written
+    const double x = sh.pos[0][lane], y = sh.pos[1][lane], z = sh.pos[2][lane];
+    for (int i = 0; i < n; ++i) {
+      if (m.warp[i] != warp) continue;
+      const DevComp& c = m.c[i];
+      const double dx = x - c.ox, dy = y - c.oy, dz = z - c.oz;
+      CompFactors f;
+      if constexpr (TIMED_) f = comp_factors(comp_at_time(c, lin[i], t), dx, dy, dz);
+      else f = comp_factors(c, dx, dy, dz);
+      m.fxy[i][lane] = f.fxy;
+      m.fz[i][lane] = f.fz;
+    }
+    __syncthreads();  // factors written
+    if (warp > 2) return 0.0;
+    double g = 0.0;
+    for (int i = 0; i < n; ++i) {
+      const double o = warp == 0 ? m.c[i].ox : warp == 1 ? m.c[i].oy : m.c[i].oz;
+      g = fma(warp < 2 ? m.fxy[i][lane] : m.fz[i][lane], q - o, g);
+    }
+    return g;
+  }
+};
 
 __device__ __forceinline__ void team_write_save(const IntegrateArgs& a, const OrbitState& s, int64_t k, int j,
                                                 double v) {
@@ -157,8 +242,8 @@ __device__ __forceinline__ void team_write_save(const IntegrateArgs& a, const Or
 
 // Takes queue positions [0, 16 g.count) in stripes, then base + atomicAdd(queue)
 // (base: all positions that this launch hands out in stripes).
-template <class TB>
-__device__ void team_loop(const IntegrateArgs& a, const MWParams& p, const Blocks& g, long long base) {
+template <class TB, class Model>
+__device__ void team_loop(const IntegrateArgs& a, const Model& pot, const Blocks& g, long long base) {
   constexpr int S = TB::S;
   constexpr double kIdle = 8.0;  // position of lanes without an orbit
   __shared__ TeamShared sh;
@@ -224,7 +309,7 @@ __device__ void team_loop(const IntegrateArgs& a, const MWParams& p, const Block
     // round, only when a lane needs it
     const bool want_f0 = fresh || (need_f0 && active);
     if (__syncthreads_or(want_f0)) {
-      const double gr = team_grad(sh, warp, lane, p, want_f0 ? yp : kIdle);
+      const double gr = pot.grad(sh, warp, lane, want_f0 ? yp : kIdle, Model::TIMED ? with_sign(s.dir, s.tau) : 0.0);
       if (want_f0) F0v = -gr;
     }
     need_f0 = false;
@@ -243,7 +328,8 @@ __device__ void team_loop(const IntegrateArgs& a, const MWParams& p, const Block
 #pragma unroll
       for (int j = 0; j < 6; ++j) F0[j] = sh.y1[j][slot];
       if (probe) is = initial_probe(a, s.y, F0);
-      const double gr = team_grad(sh, warp, lane, p, probe ? fma(is.h0 * s.dir, yv, yp) : kIdle);
+      const double gr = pot.grad(sh, warp, lane, probe ? fma(is.h0 * s.dir, yv, yp) : kIdle,
+                                 Model::TIMED ? fma(is.h0, s.dir, with_sign(s.dir, s.tau)) : 0.0);
       if (owner && !hi) {
         sh.err[j0][slot] = fma(is.h0 * s.dir, F0v, yv);
         sh.err[j1][slot] = -gr;
@@ -279,7 +365,9 @@ __device__ void team_loop(const IntegrateArgs& a, const MWParams& p, const Block
         }
         q = pair_row<TB, I, I + 1>(hi, yp, hs, Fp);
       }
-      const double f = -team_grad(sh, warp, lane, p, active ? q : kIdle);
+      constexpr double ca = TB::C[I], cb = TB::C[I + 1];
+      const double f = -pot.grad(sh, warp, lane, active ? q : kIdle,
+                                 Model::TIMED ? fma(hi ? cb : ca, hs, with_sign(s.dir, s.tau)) : 0.0);
       const double o = __shfl_xor_sync(0xffffffffu, f, kTeamLanes);
       Fv[I] = hi ? o : f;
       Fv[I + 1] = hi ? f : o;
@@ -415,7 +503,16 @@ __device__ void team_loop(const IntegrateArgs& a, const MWParams& p, const Block
 // A whole batch on teams, two blocks per SM.
 template <class TB>
 __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, MWParams p) {
-  team_loop<TB>(a, p, all_blocks(), (long long)kTeamLanes * gridDim.x);
+  __shared__ TeamMW::Shared m;
+  team_loop<TB>(a, TeamMW{p, m}, all_blocks(), (long long)kTeamLanes * gridDim.x);
+}
+
+template <class TB, bool TIMED>
+__global__ void __launch_bounds__(128, 2) k_integrate_table_team(IntegrateArgs a, const DevComp* comps, int ncomp) {
+  __shared__ typename TeamTable<TIMED>::Shared m;
+  const TeamTable<TIMED> pot{ncomp, a.lin, m};
+  pot.stage(comps);
+  team_loop<TB>(a, pot, all_blocks(), (long long)kTeamLanes * gridDim.x);
 }
 
 // Second pass of the two-pass schedule, one block of 128 threads per SM: the
@@ -423,10 +520,11 @@ __global__ void __launch_bounds__(128, 2) k_integrate_mw_team(IntegrateArgs a, M
 // thread per orbit; when their first orbits are done, all draw on one queue.
 template <class TB>
 __global__ void __launch_bounds__(128, 1) k_integrate_mw_mixed(IntegrateArgs a, MWParams p, const unsigned* teams) {
+  __shared__ TeamMW::Shared m;
   const unsigned t = min(*teams, gridDim.x - 1);
   const long long first = (long long)kTeamLanes * t;  // queue position of the longest orbit without a team
   if (blockIdx.x < t) {
-    team_loop<TB>(a, p, Blocks{t, blockIdx.x, 0}, first + 128LL * (gridDim.x - t));
+    team_loop<TB>(a, TeamMW{p, m}, Blocks{t, blockIdx.x, 0}, first + 128LL * (gridDim.x - t));
   } else {
     integrate_loop<TB>(a, MWPot{p}, Blocks{gridDim.x - t, blockIdx.x - t, first});
   }

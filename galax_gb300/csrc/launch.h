@@ -22,10 +22,13 @@ cudaError_t launch_integrate_dopri5(const IntegrateArgs& a, bool mw, const MWPar
 cudaError_t launch_integrate_dopri8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps,
                                     int ncomp, LaunchShape shape, cudaStream_t stream);
 
-// A Milky Way batch on `blocks` four-warp teams (16 orbits per block).
-cudaError_t launch_integrate_team(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream);
-cudaError_t launch_integrate_team8(const IntegrateArgs& a, const MWParams& p, int blocks, cudaStream_t stream);
-// The second pass of such a batch on `blocks` SMs, *teams (device memory) of them
+// A batch on `blocks` four-warp teams (16 orbits per block; at most
+// kTeamMaxComps components).
+cudaError_t launch_integrate_team(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                  int blocks, cudaStream_t stream);
+cudaError_t launch_integrate_team8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
+                                   int blocks, cudaStream_t stream);
+// The second pass of a Milky Way batch on `blocks` SMs, *teams (device memory) of them
 // with a team and the others with one thread per orbit. Every block requests
 // kExclusiveSmem bytes of dynamic shared memory, which it does not use, so that
 // no two share an SM.

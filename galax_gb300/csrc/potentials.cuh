@@ -204,9 +204,12 @@ static __device__ __noinline__ double plc_phi(const DevComp& c, double dx, doubl
 }
 
 // ----------------------------------------------------------- single components
-__device__ __forceinline__ void comp_grad(const DevComp& c, double x, double y, double z, double& gx, double& gy,
-                                          double& gz) {
-  const double dx = x - c.ox, dy = y - c.oy, dz = z - c.oz;
+// grad Phi = (fxy dx, fxy dy, fz dz) at the offset d from the component's centre.
+struct CompFactors {
+  double fxy, fz;
+};
+
+__device__ __forceinline__ CompFactors comp_factors(const DevComp& c, double dx, double dy, double dz) {
   if (c.kind == MIYAMOTO_NAGAI) {
     const double zb2 = fma(dz, dz, c.l2sq);
     const double izb = rsqrt(zb2);
@@ -215,10 +218,7 @@ __device__ __forceinline__ void comp_grad(const DevComp& c, double x, double y, 
     const double D2 = fma(dx, dx, fma(dy, dy, s * s));
     const double iD = rsqrt(D2);
     const double u = c.Gm * (iD * iD) * iD;
-    gx = fma(u, dx, gx);
-    gy = fma(u, dy, gy);
-    gz = fma(u * s * izb, dz, gz);
-    return;
+    return CompFactors{u, u * s * izb};
   }
   const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, TINY)));
   const double ir = rsqrt(r2);
@@ -258,9 +258,16 @@ __device__ __forceinline__ void comp_grad(const DevComp& c, double x, double y, 
       break;
     }
   }
-  gx = fma(f, dx, gx);
-  gy = fma(f, dy, gy);
-  gz = fma(f, dz, gz);
+  return CompFactors{f, f};
+}
+
+__device__ __forceinline__ void comp_grad(const DevComp& c, double x, double y, double z, double& gx, double& gy,
+                                          double& gz) {
+  const double dx = x - c.ox, dy = y - c.oy, dz = z - c.oz;
+  const CompFactors f = comp_factors(c, dx, dy, dz);
+  gx = fma(f.fxy, dx, gx);
+  gy = fma(f.fxy, dy, gy);
+  gz = fma(f.fz, dz, gz);
 }
 
 __device__ __forceinline__ double comp_phi(const DevComp& c, double x, double y, double z) {

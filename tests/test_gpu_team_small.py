@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("method", [5, 8])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 2433, 9728])
-@pytest.mark.parametrize("case", ["adaptive", "constant", "pid_dtmin", "host_saves", "order"])
+@pytest.mark.parametrize("case", ["adaptive", "constant", "pid_dtmin", "host_saves", "order", "mw2022", "bovy", "linear",
+                                  "sixteen"])
 def test_small_batches_match_one_thread_per_orbit(method, n, case):
     import torch
 
@@ -17,10 +18,21 @@ def test_small_batches_match_one_thread_per_orbit(method, n, case):
     from galax_gb300 import _lib
     from galax_gb300 import dynamics as D
 
-    if n > 100 and case not in ("adaptive", "constant"):
+    if n > 100 and case not in ("adaptive", "constant", "mw2022"):
         pytest.skip("the sizes that matter to these are the small ones")
     L = _lib.load()
-    mw = gx.MilkyWayPotential()
+    if case == "mw2022":
+        mw = gx.MilkyWayPotential2022()
+    elif case == "bovy":  # a disk, an incomplete gamma function, a halo
+        mw = gx.BovyMWPotential2014()
+    elif case == "linear":
+        mw = gx.MilkyWayPotential(halo={"m": gx.LinearParameter(slope=6e8, point_time=10.0, point_value=5.4e11)})
+    elif case == "sixteen":  # the largest table that teams take, components off the centre
+        mw = gx.CompositePotential([gx.MilkyWayPotential()] + [
+            gx.PlummerPotential(m_tot=1e9 * (k + 1), r_s=0.5, origin=(k, -k, 0.5 * k)) if k % 2 else
+            gx.IsochronePotential(m_tot=1e9, r_s=1.0 + k, origin=(0.0, k, 1.0)) for k in range(12)])
+    else:
+        mw = gx.MilkyWayPotential()
     rng = np.random.default_rng(n)
     x = rng.normal(size=(n, 3)) * 6.0
     y0 = np.concatenate([x, rng.normal(size=(n, 3)) * 0.12], axis=1)
