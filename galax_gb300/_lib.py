@@ -111,6 +111,8 @@ SIGNATURES = {
                                      C.c_int64, _DP, C.c_void_p, C.c_void_p]),
     "gal_adjoint_workspace_size": (C.c_int, [C.c_void_p, C.POINTER(SolverConfig), C.c_double, C.c_double,
                                              C.c_int32, C.c_int64, C.POINTER(C.c_size_t)]),
+    "gal_adjoint_workspace_size_stored": (C.c_int, [C.c_void_p, C.POINTER(SolverConfig), C.c_double, C.c_double,
+                                                    C.c_int32, C.c_int64, C.c_size_t, C.POINTER(C.c_size_t)]),
     "gal_adjoint": (C.c_int, [C.c_void_p, C.POINTER(SolverConfig), _DP, C.c_double, C.c_double, _DP, _DP, _DP, _DP,
                               _DP, C.c_int32, C.c_int64, _VP, C.c_size_t, C.c_void_p]),
     "gal_stream_workspace_size": (C.c_int, [C.c_void_p, C.POINTER(StreamConfig), C.c_int32,

@@ -43,6 +43,20 @@ class AdjointResult:
 
 
 _WS = Workspace()
+# At most this much scratch for stored stages (12 GB); what a call needs beyond the
+# kept workspace's bound (256 MB) it allocates for itself.
+STORED_STAGES_MAX = 12 << 30
+_KEPT_MAX = 256 << 20
+
+
+def _scratch(nbytes: int):
+    torch = _torch()
+    if nbytes <= _KEPT_MAX:
+        return _WS.get(nbytes)
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    except torch.cuda.OutOfMemoryError:
+        return None
 
 
 def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None, stream=None):
@@ -55,9 +69,14 @@ def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None,
     L = _lib.load()
     h = pot.handle()
     nb = C.c_size_t()
-    _lib.check(L.gal_adjoint_workspace_size(h, C.byref(cfg), float(t0), float(t1), int(k_ckpt), n, C.byref(nb)),
-               "gal_adjoint_workspace_size")
-    ws = _WS.get(nb.value)
+    _lib.check(L.gal_adjoint_workspace_size_stored(h, C.byref(cfg), float(t0), float(t1), int(k_ckpt), n,
+                                                   STORED_STAGES_MAX, C.byref(nb)),
+               "gal_adjoint_workspace_size_stored")
+    ws = _scratch(nb.value)
+    if ws is None:  # no room for stored stages: checkpoints alone
+        _lib.check(L.gal_adjoint_workspace_size(h, C.byref(cfg), float(t0), float(t1), int(k_ckpt), n, C.byref(nb)),
+                   "gal_adjoint_workspace_size")
+        ws = _WS.get(nb.value)
     yT = torch.empty((6, n), dtype=torch.float64, device="cuda")
     gy = torch.empty((6, n), dtype=torch.float64, device="cuda")
     ncomp = len(pot.components())

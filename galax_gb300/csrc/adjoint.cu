@@ -30,6 +30,7 @@
 
 #include "handle.h"
 #include "integrate.cuh"
+#include "nystrom.cuh"
 #include "vjp.cuh"
 
 namespace gal {
@@ -162,6 +163,231 @@ __global__ void __launch_bounds__(128) k_adjoint(AdjointArgs a, Pot pot, const D
   for (int i = 0; i < ncomp * NP; ++i) a.gp_orbit[(int64_t)i * n + o] = gp[i];
 }
 
+// ----------------------------------------------------------------- Milky Way
+// The static Milky Way's adjoint with stored stages. It is FP64-bound, so it does
+// each evaluation once: the forward step keeps, for every stage, the position
+// and what its gradient was made of (radius, logarithm, reciprocals: 10 doubles),
+// and the reverse sweep forms the Hessian-vector product and the parameter terms
+// from these. Steps are in Nystrom form both ways: with
+// gbar_l = -h [bbar_l h lx + b_l lv + h sum_{i>l} abar_il Xbar_i],
+//   Xbar_i = H(X_i) gbar_i,   lx += sum_i Xbar_i,   lv += h lx + h sum_i c_i Xbar_i,
+//   dL/dtheta += sum_i gbar_i . (dg/dtheta)(X_i).
+// The scratch holds the stages of `seg` steps; longer spans are cut into such
+// segments, and all but the last are integrated a second time from their first
+// state. FP64 instructions per Dopri8 step: 2,960 (4,240 with segments), where
+// k_adjoint takes 8,260 (three forward evaluations and four separate components).
+// 16,384 orbits, 500 steps: 143.5 -> 48.0 ms.
+constexpr int kStageDoubles = 10;
+
+struct StoredArgs {
+  const double* y0;
+  const double* lambda;
+  const double* target;
+  double* yT;
+  double* grad_y0;
+  const double* ts;
+  double* ckpt;      // [ceil(nsteps / seg)][6][n]
+  double* stages;    // [seg][S][kStageDoubles][n]
+  double* gp_orbit;  // [12][n]
+  int64_t nsteps, seg, n;
+};
+
+// Gradient at X; q: ir, L, 1/(r + r_s) of halo, bulge, nucleus, 1/sqrt(z^2 + b^2), 1/D.
+__device__ __forceinline__ void mw_stage(const MWParams& p, const double* X, double* q, double* g) {
+  double r;
+  const double ir = mw_ir(X[0], X[1], X[2], r);
+  const double dh = p.rs_h + r, db = r + p.rs_b, dn = r + p.rs_n;
+  const double bn = db * dn;
+  const double iP = 1.0 / (dh * bn);
+  const double ih = iP * dh;
+  const double idh = iP * bn, idb = ih * dn, idn = ih * db;
+  const double L = mw_halo_log(p, r);
+  const double zb2 = fma(X[2], X[2], p.b2_d);
+  const double izb = rsqrt(zb2);
+  const double s = fma(zb2, izb, p.a_d);
+  const double iD = rsqrt(fma(s, s, fma(X[0], X[0], X[1] * X[1])));
+  const double u = p.Gm_d * (iD * iD) * iD;
+  const double f = p.Gm_h * (ir * ir) * fma(L, ir, -idh) + ir * fma(p.Gm_b, idb * idb, p.Gm_n * (idn * idn));
+  g[0] = (u + f) * X[0];
+  g[1] = (u + f) * X[1];
+  g[2] = fma(u * s, izb, f) * X[2];
+  q[0] = ir;
+  q[1] = L;
+  q[2] = idh;
+  q[3] = idb;
+  q[4] = idn;
+  q[5] = izb;
+  q[6] = iD;
+}
+
+// H(X) w, and the parameter sums of g . w up to constant factors (see the end of
+// the kernel): disk m, a, b; halo m, r_s; bulge m, r_s; nucleus m, r_s.
+__device__ __forceinline__ void mw_stage_vjp(const MWParams& p, const double* X, const double* q, const double* w,
+                                             double* Hw, double* gp) {
+  const double ir = q[0], L = q[1], idh = q[2], idb = q[3], idn = q[4], izb = q[5], iD = q[6];
+  const double xw = fma(X[0], w[0], fma(X[1], w[1], X[2] * w[2]));
+  const double ir2 = ir * ir;
+  const double idh2 = idh * idh;
+  const double gh = p.Gm_h * ir2 * fma(L, ir, -idh);
+  const double gb = p.Gm_b * ir * (idb * idb), gn = p.Gm_n * ir * (idn * idn);
+  const double gpr = ir2 * fma(p.Gm_h * ir, idh2, -3.0 * gh) -
+                     fma(gb, fma(2.0 * ir, idb, ir2), gn * fma(2.0 * ir, idn, ir2));
+  gp[3] = fma(gh, xw, gp[3]);
+  gp[4] = fma(ir * idh2, xw, gp[4]);
+  const double bw = gb * xw, nw = gn * xw;
+  gp[5] += bw;
+  gp[6] = fma(bw, idb, gp[6]);
+  gp[7] += nw;
+  gp[8] = fma(nw, idn, gp[8]);
+  const double iD2 = iD * iD;
+  const double u = p.Gm_d * iD2 * iD;
+  const double w5 = 3.0 * u * iD2;
+  const double s = fma(fma(X[2], X[2], p.b2_d), izb, p.a_d);
+  const double zi = X[2] * izb;
+  const double vz = zi * s;
+  const double vw = fma(X[0], w[0], fma(X[1], w[1], vz * w[2]));
+  const double izb2 = izb * izb;
+  const double t = w5 * vw, ts = t * s;
+  const double uz = u * w[2], uzi = uz * zi;
+  gp[0] = fma(u, vw, gp[0]);
+  gp[1] += uzi - ts;
+  gp[2] -= fma(ts, izb, p.a_d * uzi * izb2);
+  const double d = u + (gh + (gb + gn));
+  const double k = fma(gpr, xw, -t);
+  Hw[0] = fma(d, w[0], k * X[0]);
+  Hw[1] = fma(d, w[1], k * X[1]);
+  Hw[2] = fma(d, w[2], fma(gpr * xw, X[2], fma(-t, vz, p.a_d * p.b2_d * (izb2 * izb) * uz)));
+}
+
+template <class TB>
+__global__ void __launch_bounds__(32) k_adjoint_mw(StoredArgs a, MWParams p, const DevComp* comps) {
+  constexpr int S = TB::S;
+  const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (o >= a.n) return;
+  const int64_t n = a.n;
+  double x[3], v[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    x[j] = a.y0[j * n + o];
+    v[j] = a.y0[(3 + j) * n + o];
+  }
+  // one step from (x, v); its stages go to scratch row `row` (none if < 0)
+  auto step = [&](int64_t k, int64_t row) {
+    const double h = a.ts[k + 1] - a.ts[k];
+    double g[S][3];
+    static_for<0, S>([&](auto i) {
+      constexpr int I = decltype(i)::value;
+      if constexpr (kNystrom<TB>.used[I]) {
+        double X[3], q[7];
+        if constexpr (I == 0) {
+#pragma unroll
+          for (int j = 0; j < 3; ++j) X[j] = x[j];
+        } else {
+          nystrom_stage<TB, I>(x, v, h, g, X);
+        }
+        mw_stage(p, X, q, g[I]);
+        if (row >= 0) {
+          double* st = a.stages + ((row * S + I) * kStageDoubles) * n + o;
+#pragma unroll
+          for (int j = 0; j < 3; ++j) st[j * n] = X[j];
+#pragma unroll
+          for (int j = 0; j < 7; ++j) st[(3 + j) * n] = q[j];
+        }
+      }
+    });
+    nystrom_end<TB>(x, v, h, g);
+  };
+  const int64_t nseg = (a.nsteps + a.seg - 1) / a.seg;
+  const int64_t last = (nseg - 1) * a.seg;
+  for (int64_t k = 0; k < a.nsteps; ++k) {
+    if (k % a.seg == 0 && k < last) {
+      double* c = a.ckpt + (k / a.seg) * 6 * n + o;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        c[j * n] = x[j];
+        c[(3 + j) * n] = v[j];
+      }
+    }
+    step(k, k - last);
+  }
+  double lx[3], lv[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    a.yT[j * n + o] = x[j];
+    a.yT[(3 + j) * n + o] = v[j];
+    lx[j] = a.lambda ? a.lambda[j * n + o] : 2.0 * (x[j] - a.target[j * n + o]);
+    lv[j] = a.lambda ? a.lambda[(3 + j) * n + o] : 2.0 * (v[j] - a.target[(3 + j) * n + o]);
+  }
+  double gp[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int64_t sgi = nseg - 1; sgi >= 0; --sgi) {
+    const int64_t k0 = sgi * a.seg;
+    const int64_t k1 = k0 + a.seg < a.nsteps ? k0 + a.seg : a.nsteps;
+    if (sgi != nseg - 1) {
+      const double* c = a.ckpt + sgi * 6 * n + o;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        x[j] = c[j * n];
+        v[j] = c[(3 + j) * n];
+      }
+      for (int64_t k = k0; k < k1; ++k) step(k, k - k0);
+    }
+    for (int64_t k = k1 - 1; k >= k0; --k) {
+      const double h = a.ts[k + 1] - a.ts[k];
+      double G[S][3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const double hl = h * lx[j], l = lv[j];
+        static_for<0, S>([&](auto i) {
+          constexpr int I = decltype(i)::value;
+          constexpr double cx = kNystrom<TB>.b[I], cv = TB::B[I];
+          if constexpr (cx != 0.0 && cv != 0.0) G[I][j] = fma(cx, hl, cv * l);
+          else if constexpr (cx != 0.0) G[I][j] = cx * hl;
+          else if constexpr (cv != 0.0) G[I][j] = cv * l;
+          else G[I][j] = 0.0;
+        });
+        lv[j] += hl;
+      }
+      static_for<0, S>([&](auto r) {
+        constexpr int I = S - 1 - decltype(r)::value;
+        if constexpr (kNystrom<TB>.used[I]) {
+          const double* st = a.stages + (((k - k0) * S + I) * kStageDoubles) * n + o;
+          double X[3], q[7], w[3], Xb[3];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) X[j] = st[j * n];
+#pragma unroll
+          for (int j = 0; j < 7; ++j) q[j] = st[(3 + j) * n];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) w[j] = -h * G[I][j];
+          mw_stage_vjp(p, X, q, w, Xb, gp);
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            lx[j] += Xb[j];
+            constexpr double ci = TB::C[I];
+            const double E = h * Xb[j];
+            if constexpr (ci != 0.0) lv[j] = fma(ci, E, lv[j]);
+            static_for<0, I>([&](auto l) {
+              constexpr int L = decltype(l)::value;
+              constexpr double c = kNystrom<TB>.a[I][L];
+              if constexpr (c != 0.0) G[L][j] = fma(c, E, G[L][j]);
+            });
+          }
+        }
+      });
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    a.grad_y0[j * n + o] = lx[j];
+    a.grad_y0[(3 + j) * n + o] = lv[j];
+  }
+  const double out[12] = {gp[0] * comps[0].inv_m, gp[1], comps[0].l2 * gp[2],
+                          gp[3] * comps[1].inv_m, -p.Gm_h * p.irs_h * gp[4], 0.0,
+                          gp[5] * comps[2].inv_m, -2.0 * gp[6], 0.0,
+                          gp[7] * comps[3].inv_m, -2.0 * gp[8], 0.0};
+#pragma unroll
+  for (int i = 0; i < 12; ++i) a.gp_orbit[i * n + o] = out[i];
+}
+
 // grad_params[p] = sum over orbits of gp_orbit[p][:], in a fixed order.
 __global__ void k_reduce_rows(const double* __restrict__ in, int64_t n, double* __restrict__ out) {
   __shared__ double red[256];
@@ -229,6 +455,11 @@ static AdjLayout adj_layout(int ncomp, int np, const std::vector<double>& ts, in
   return L;
 }
 
+// Scratch of one step's stored stages (k_adjoint_mw).
+static size_t stored_step_bytes(int method, int64_t n) {
+  return sizeof(double) * (size_t)((method == 8 ? Dopri8::S : Dopri5::S) * kStageDoubles) * (size_t)n;
+}
+
 }  // namespace gal
 
 using namespace gal;
@@ -244,6 +475,21 @@ gal_status gal_adjoint_workspace_size(const gal_potential* pot, const gal_solver
     if (!time_grid(t0, t1, cfg->dt0, cfg->max_steps, ts))
       return fail(GAL_ERR_INVALID_ARGUMENT, "t0 and t1 must be finite and at most max_steps steps of dt0 apart");
     *bytes = adj_layout(pot->n, time_dependent(pot) ? 6 : 3, ts, k_ckpt, n).total;
+    return GAL_OK;
+  });
+}
+
+gal_status gal_adjoint_workspace_size_stored(const gal_potential* pot, const gal_solver_config* cfg, double t0,
+                                             double t1, int32_t k_ckpt, int64_t n, size_t max_extra, size_t* bytes) {
+  return no_throw([&]() -> gal_status {
+    const gal_status st = gal_adjoint_workspace_size(pot, cfg, t0, t1, k_ckpt, n, bytes);
+    if (st != GAL_OK || !pot->is_mw || n == 0) return st;
+    std::vector<double> ts;
+    time_grid(t0, t1, cfg->dt0, cfg->max_steps, ts);
+    const size_t per_step = stored_step_bytes(cfg->method, n);
+    size_t steps = max_extra / per_step;
+    if (steps > ts.size() - 1) steps = ts.size() - 1;
+    *bytes += steps * per_step;
     return GAL_OK;
   });
 }
@@ -288,6 +534,37 @@ gal_status gal_adjoint(const gal_potential* pot, const gal_solver_config* cfg, c
     a.k_ckpt = k_ckpt;
     a.n = n;
     a.lin = pot->d_lin;
+    // Stored stages when the workspace has room for at least eight steps of them
+    // (or all): below that, and for other tables, checkpoints every k_ckpt steps.
+    if (pot->is_mw) {
+      int64_t seg = (int64_t)((workspace_bytes - L.total) / stored_step_bytes(cfg->method, n));
+      if (seg > L.nsteps) seg = L.nsteps;
+      const int64_t nseg = seg > 0 ? (L.nsteps + seg - 1) / seg : 0;
+      const size_t states = (L.gp - L.ckpt) / (6 * sizeof(double) * (size_t)n);  // the checkpoint and segment areas
+      if ((seg >= 8 || seg == L.nsteps) && (size_t)nseg <= states) {
+        StoredArgs b{};
+        b.y0 = y0;
+        b.lambda = lambda;
+        b.target = target;
+        b.yT = yT;
+        b.grad_y0 = grad_y0;
+        b.ts = a.ts;
+        b.ckpt = a.ckpt;
+        b.stages = reinterpret_cast<double*>(ws + L.total);
+        b.gp_orbit = a.gp_orbit;
+        b.nsteps = L.nsteps;
+        b.seg = seg;
+        b.n = n;
+        const unsigned blocks = (unsigned)((n + 31) / 32);  // one warp each, for an even spread over the SMs
+        if (cfg->method == 8) k_adjoint_mw<Dopri8><<<blocks, 32, 0, s>>>(b, pot->mw, pot->d_comps);
+        else k_adjoint_mw<Dopri5><<<blocks, 32, 0, s>>>(b, pot->mw, pot->d_comps);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return cuda_fail(e, "adjoint kernel launch (stored stages)");
+        k_reduce_rows<<<12, 256, 0, s>>>(a.gp_orbit, n, grad_params);
+        e = cudaGetLastError();
+        return e == cudaSuccess ? GAL_OK : cuda_fail(e, "adjoint reduction launch");
+      }
+    }
     const int block = 64;
     const unsigned grid = (unsigned)((n + block - 1) / block);
     if (timed) {

@@ -294,6 +294,12 @@ GAL_API gal_status gal_set_table_lanes(int32_t lanes);
 /* Scratch bytes gal_adjoint needs for n orbits with checkpoints every k_ckpt steps. */
 GAL_API gal_status gal_adjoint_workspace_size(const gal_potential* pot, const gal_solver_config* cfg, double t0, double t1,
                                       int32_t k_ckpt, int64_t n, size_t* bytes);
+/* The same, plus room for the stages of as many steps as max_extra bytes hold
+ * (static Milky Way only: 1,040 bytes per orbit and Dopri8 step, 560 for Dopri5).
+ * With such a workspace gal_adjoint stores the forward pass's stages instead of
+ * evaluating them again in the reverse sweep; the gradients agree to rounding. */
+GAL_API gal_status gal_adjoint_workspace_size_stored(const gal_potential* pot, const gal_solver_config* cfg, double t0,
+                                             double t1, int32_t k_ckpt, int64_t n, size_t max_extra, size_t* bytes);
 
 /* Discrete adjoint of the constant-step map y(t0) -> y(t1) (cfg->adaptive must be
  * 0; step cfg->dt0) for terminal cotangents: given lambda = dL/dy(t1) [6][n],
