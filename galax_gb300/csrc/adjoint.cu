@@ -192,73 +192,6 @@ struct StoredArgs {
   int64_t nsteps, seg, n;
 };
 
-// Gradient at X; q: ir, L, 1/(r + r_s) of halo, bulge, nucleus, 1/sqrt(z^2 + b^2), 1/D.
-__device__ __forceinline__ void mw_stage(const MWParams& p, const double* X, double* q, double* g) {
-  double r;
-  const double ir = mw_ir(X[0], X[1], X[2], r);
-  const double dh = p.rs_h + r, db = r + p.rs_b, dn = r + p.rs_n;
-  const double bn = db * dn;
-  const double iP = 1.0 / (dh * bn);
-  const double ih = iP * dh;
-  const double idh = iP * bn, idb = ih * dn, idn = ih * db;
-  const double L = mw_halo_log(p, r);
-  const double zb2 = fma(X[2], X[2], p.b2_d);
-  const double izb = rsqrt(zb2);
-  const double s = fma(zb2, izb, p.a_d);
-  const double iD = rsqrt(fma(s, s, fma(X[0], X[0], X[1] * X[1])));
-  const double u = p.Gm_d * (iD * iD) * iD;
-  const double f = p.Gm_h * (ir * ir) * fma(L, ir, -idh) + ir * fma(p.Gm_b, idb * idb, p.Gm_n * (idn * idn));
-  g[0] = (u + f) * X[0];
-  g[1] = (u + f) * X[1];
-  g[2] = fma(u * s, izb, f) * X[2];
-  q[0] = ir;
-  q[1] = L;
-  q[2] = idh;
-  q[3] = idb;
-  q[4] = idn;
-  q[5] = izb;
-  q[6] = iD;
-}
-
-// H(X) w, and the parameter sums of g . w up to constant factors (see the end of
-// the kernel): disk m, a, b; halo m, r_s; bulge m, r_s; nucleus m, r_s.
-__device__ __forceinline__ void mw_stage_vjp(const MWParams& p, const double* X, const double* q, const double* w,
-                                             double* Hw, double* gp) {
-  const double ir = q[0], L = q[1], idh = q[2], idb = q[3], idn = q[4], izb = q[5], iD = q[6];
-  const double xw = fma(X[0], w[0], fma(X[1], w[1], X[2] * w[2]));
-  const double ir2 = ir * ir;
-  const double idh2 = idh * idh;
-  const double gh = p.Gm_h * ir2 * fma(L, ir, -idh);
-  const double gb = p.Gm_b * ir * (idb * idb), gn = p.Gm_n * ir * (idn * idn);
-  const double gpr = ir2 * fma(p.Gm_h * ir, idh2, -3.0 * gh) -
-                     fma(gb, fma(2.0 * ir, idb, ir2), gn * fma(2.0 * ir, idn, ir2));
-  gp[3] = fma(gh, xw, gp[3]);
-  gp[4] = fma(ir * idh2, xw, gp[4]);
-  const double bw = gb * xw, nw = gn * xw;
-  gp[5] += bw;
-  gp[6] = fma(bw, idb, gp[6]);
-  gp[7] += nw;
-  gp[8] = fma(nw, idn, gp[8]);
-  const double iD2 = iD * iD;
-  const double u = p.Gm_d * iD2 * iD;
-  const double w5 = 3.0 * u * iD2;
-  const double s = fma(fma(X[2], X[2], p.b2_d), izb, p.a_d);
-  const double zi = X[2] * izb;
-  const double vz = zi * s;
-  const double vw = fma(X[0], w[0], fma(X[1], w[1], vz * w[2]));
-  const double izb2 = izb * izb;
-  const double t = w5 * vw, ts = t * s;
-  const double uz = u * w[2], uzi = uz * zi;
-  gp[0] = fma(u, vw, gp[0]);
-  gp[1] += uzi - ts;
-  gp[2] -= fma(ts, izb, p.a_d * uzi * izb2);
-  const double d = u + (gh + (gb + gn));
-  const double k = fma(gpr, xw, -t);
-  Hw[0] = fma(d, w[0], k * X[0]);
-  Hw[1] = fma(d, w[1], k * X[1]);
-  Hw[2] = fma(d, w[2], fma(gpr * xw, X[2], fma(-t, vz, p.a_d * p.b2_d * (izb2 * izb) * uz)));
-}
-
 template <class TB>
 __global__ void __launch_bounds__(32) k_adjoint_mw(StoredArgs a, MWParams p, const DevComp* comps) {
   constexpr int S = TB::S;
@@ -380,10 +313,8 @@ __global__ void __launch_bounds__(32) k_adjoint_mw(StoredArgs a, MWParams p, con
     a.grad_y0[j * n + o] = lx[j];
     a.grad_y0[(3 + j) * n + o] = lv[j];
   }
-  const double out[12] = {gp[0] * comps[0].inv_m, gp[1], comps[0].l2 * gp[2],
-                          gp[3] * comps[1].inv_m, -p.Gm_h * p.irs_h * gp[4], 0.0,
-                          gp[5] * comps[2].inv_m, -2.0 * gp[6], 0.0,
-                          gp[7] * comps[3].inv_m, -2.0 * gp[8], 0.0};
+  double out[12];
+  mw_param_grads(p, comps, gp, out);
 #pragma unroll
   for (int i = 0; i < 12; ++i) a.gp_orbit[i * n + o] = out[i];
 }

@@ -92,6 +92,24 @@ __device__ __forceinline__ void stage_comps(const DevComp* comps, int ncomp, Dev
   __syncthreads();
 }
 
+// Hessian of the host (xx xy xz yy yz zz).
+template <bool MW>
+__device__ __forceinline__ void host_hessian(const DevComp* comps, int ncomp, const MWParams& mwp, const double* Y,
+                                             double* H) {
+  if constexpr (MW) {
+    mw_hessian(mwp, Y[0], Y[1], Y[2], H);
+  } else {
+    double F[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int c = 0; c < ncomp; ++c) comp_hessian(comps[c], Y[0], Y[1], Y[2], F);
+    H[0] = F[0];
+    H[1] = F[1];
+    H[2] = F[2];
+    H[3] = F[4];
+    H[4] = F[5];
+    H[5] = F[8];
+  }
+}
+
 // Particle field: host potential plus the progenitor's Plummer sphere at q,
 // summed in the order of the four-warp particle kernel: partial sum w
 // (w = 0..3) holds components w, w + 4, ... and partial 3 also the Plummer
@@ -227,112 +245,6 @@ __device__ __forceinline__ void team_step(const DevComp* comps, int ncomp, doubl
   __syncthreads();
 }
 
-// team_step for a Milky Way host: the gradient split as in the integrators'
-// four-warp teams (warp 0: radius and shared reciprocal, warp 1: NFW log,
-// warp 3: disk; mw_* pieces), combined on lanes 0-2 of warp 0. The NFW log,
-// the longest chain, no longer shares a warp with the rest of its component.
-template <class TB>
-__device__ __forceinline__ void team_step_mw(const MWParams& p, double hs, double* Qk, double* sy,
-                                             double (*sF)[6], double* sY, double* sw, int warp, int lane) {
-  constexpr int S = TB::S;
-  const bool comb = warp == 0 && lane < 6;
-  // sw: [0] ir, [1] inv_dh, [2] inv_db2, [3] inv_dn2, [4] L, [5] u, [6] us, [7] izb
-  auto slope = [&](int I) {
-    __syncthreads();  // sY complete
-    if (lane == 0) {
-      const double x = sY[0], y = sY[1], z = sY[2];
-      if (warp == 0) {
-        double r;
-        const double ir = mw_ir(x, y, z, r);
-        const MWRecip c = mw_recip(p, r);
-        sw[0] = ir;
-        sw[1] = c.inv_dh;
-        sw[2] = c.inv_db2;
-        sw[3] = c.inv_dn2;
-      } else if (warp == 1) {
-        double r;
-        mw_ir(x, y, z, r);
-        sw[4] = mw_halo_log(p, r);
-      } else if (warp == 3) {
-        const MWDisk d = mw_disk(p, x, y, z);
-        sw[5] = d.u;
-        sw[6] = d.us;
-        sw[7] = d.izb;
-      }
-    }
-    __syncthreads();  // pieces complete
-    if (comb) {
-      double f;
-      if (lane < 3) {
-        f = sY[lane + 3];
-      } else {
-        const MWRecip c{sw[1], sw[2], sw[3]};
-        const double fr = mw_f(p, sw[0], sw[4], c);
-        const int j = lane - 3;
-        const double g = (j == 2) ? fma(sw[6], sw[7], fr) * sY[2] : (sw[5] + fr) * sY[j];
-        f = -g;
-      }
-      sF[I][lane] = f;
-      if (Qk && lane < 3) Qk[3 * I + lane] = sY[lane];
-    }
-  };
-  if (comb) sY[lane] = sy[lane];
-  slope(0);
-  static_for<1, S>([&](auto i) {
-    constexpr int I = decltype(i)::value;
-    __syncthreads();  // sF[I-1] written, sY free for reuse
-    if (comb) {
-      double acc = 0.0;
-      bool first = true;
-      static_for<0, I>([&](auto l) {
-        constexpr int L = decltype(l)::value;
-        constexpr double c = TB::A[I][L];
-        if constexpr (c != 0.0) {
-          acc = first ? c * sF[L][lane] : fma(c, sF[L][lane], acc);
-          first = false;
-        }
-      });
-      sY[lane] = fma(hs, acc, sy[lane]);
-    }
-    slope(I);
-  });
-  __syncthreads();
-  if (comb) {
-    double acc = 0.0;
-    bool first = true;
-    static_for<0, S>([&](auto l) {
-      constexpr int L = decltype(l)::value;
-      constexpr double c = TB::B[L];
-      if constexpr (c != 0.0) {
-        acc = first ? c * sF[L][lane] : fma(c, sF[L][lane], acc);
-        first = false;
-      }
-    });
-    sy[lane] = fma(hs, acc, sy[lane]);
-  }
-  __syncthreads();
-}
-
-template <class TB>
-__global__ void __launch_bounds__(128) k_stream_progenitor_mw(StreamDev a, MWParams p) {
-  __shared__ double sy[6], sY[6], sF[TB::S][6], sw[8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < 6) {
-    sy[threadIdx.x] = a.w_now[threadIdx.x];
-    a.B[threadIdx.x] = sy[threadIdx.x];
-  }
-  __syncthreads();
-  for (int64_t k = 0; k < a.n_rel; ++k) {
-    team_step_mw<TB>(p, -a.dt, a.Qb ? a.Qb + k * TB::S * 3 : nullptr, sy, sF, sY, sw, warp, lane);
-    if (threadIdx.x < 6) a.B[(k + 1) * 6 + threadIdx.x] = sy[threadIdx.x];
-  }
-  if (threadIdx.x < 6) a.P[threadIdx.x] = sy[threadIdx.x];
-  for (int64_t k = 0; k < a.n_rel; ++k) {
-    team_step_mw<TB>(p, a.dt, a.Q + k * TB::S * 3, sy, sF, sY, sw, warp, lane);
-    if (threadIdx.x < 6) a.P[(k + 1) * 6 + threadIdx.x] = sy[threadIdx.x];
-  }
-}
-
 template <class TB>
 __global__ void __launch_bounds__(128) k_stream_progenitor_team(StreamDev a, const DevComp* comps) {
   __shared__ DevComp s_comps[kAdjMaxComps];
@@ -356,114 +268,18 @@ __global__ void __launch_bounds__(128) k_stream_progenitor_team(StreamDev a, con
 }
 
 
-// Particles on teams of four warps: block b integrates particles 32b .. 32b+31
-// (one per lane). Warps 0-2 own state components (w, w+3) of their lane's
-// particle and form the stage states; every warp evaluates its share of the
-// host components (component c on warp c % 4) and warp 3 also the progenitor's
-// Plummer sphere; warps 0-2 then sum the four partial gradients in warp order.
-// A lane joins when the global step reaches its release step. Writes the final
-// states and either the checkpoints or the stored stage positions.
-template <class TB>
-__global__ void __launch_bounds__(128) k_stream_particles_team(StreamDev a, const DevComp* comps) {
-  __shared__ DevComp s_comps[kAdjMaxComps];
-  __shared__ double sY[3][32], sg[4][3][32];
-  stage_comps(comps, a.ncomp, s_comps);
-  constexpr int S = TB::S;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t p = (int64_t)blockIdx.x * 32 + lane;
-  const int64_t n = a.np;
-  const bool valid = p < n;
-  const int64_t rp = valid ? (p >> 1) : LLONG_MAX;
-  const int64_t rmin = ((int64_t)blockIdx.x * 32) >> 1;
-  const bool own = warp < 3;
-  const int j0 = warp, j1 = warp + 3;  // state components owned by warps 0-2
-  const int K = a.k_ckpt;
-  double y0 = 0.0, y1 = 0.0;  // this warp's two components of the lane's particle
-  if (own) {  // lanes past the last particle follow a circular-ish orbit at 8 kpc
-    y0 = valid ? a.ics[j0 * n + p] : (j0 == 0 ? 8.0 : 0.0);
-    y1 = valid ? a.ics[j1 * n + p] : (j1 == 4 ? 0.2 : 0.0);
-  }
-  for (int64_t k = rmin; k < a.n_rel; ++k) {
-    const bool act = valid && k >= rp;
-    if (own && act && a.ckpt && (k == rp || k % K == 0)) {
-      const int64_t g = k / K;
-      a.ckpt[(g * 6 + j0) * n + p] = y0;
-      a.ckpt[(g * 6 + j1) * n + p] = y1;
-    }
-    const double* Qk = a.Q + k * S * 3;
-    double F0[S] = {}, F1[S] = {};  // this warp's components of the stage slopes
-    static_for<0, S>([&](auto i) {
-      constexpr int I = decltype(i)::value;
-      double Y0 = y0, Y1 = y1;
-      if (own && I > 0) {
-        double c0 = 0.0, c1 = 0.0;
-        bool first = true;
-        static_for<0, I>([&](auto l) {
-          constexpr int L = decltype(l)::value;
-          constexpr double c = TB::A[I][L];
-          if constexpr (c != 0.0) {
-            c0 = first ? c * F0[L] : fma(c, F0[L], c0);
-            c1 = first ? c * F1[L] : fma(c, F1[L], c1);
-            first = false;
-          }
-        });
-        Y0 = fma(a.dt, c0, y0);
-        Y1 = fma(a.dt, c1, y1);
-      }
-      if (own) {
-        sY[j0][lane] = Y0;
-        if (a.Ys && act) a.Ys[stage_idx(k, I, j0, p, S, 3)] = Y0;
-      }
-      __syncthreads();
-      const double x0 = sY[0][lane], x1 = sY[1][lane], x2 = sY[2][lane];
-      double gx = 0.0, gy = 0.0, gz = 0.0;
-      for (int c = warp; c < a.ncomp; c += 4) comp_grad(s_comps[c], x0, x1, x2, gx, gy, gz);
-      if (warp == 3) {  // the progenitor's Plummer sphere at its stage position
-        const double d0 = x0 - Qk[3 * I], d1 = x1 - Qk[3 * I + 1], d2 = x2 - Qk[3 * I + 2];
-        const double r2 = fma(d0, d0, fma(d1, d1, fma(d2, d2, TINY)));
-        const double is = rsqrt(r2 + a.b2);
-        const double f = a.GMp * (is * is) * is;
-        gx = fma(f, d0, gx);
-        gy = fma(f, d1, gy);
-        gz = fma(f, d2, gz);
-      }
-      sg[warp][0][lane] = gx;
-      sg[warp][1][lane] = gy;
-      sg[warp][2][lane] = gz;
-      __syncthreads();
-      if (own) {
-        F0[I] = Y1;  // dq/dt = p
-        F1[I] = -(((sg[0][j0][lane] + sg[1][j0][lane]) + sg[2][j0][lane]) + sg[3][j0][lane]);
-      }
-    });
-    if (own && act) {
-      double c0 = 0.0, c1 = 0.0;
-      bool first = true;
-      static_for<0, S>([&](auto l) {
-        constexpr int L = decltype(l)::value;
-        constexpr double c = TB::B[L];
-        if constexpr (c != 0.0) {
-          c0 = first ? c * F0[L] : fma(c, F0[L], c0);
-          c1 = first ? c * F1[L] : fma(c, F1[L], c1);
-          first = false;
-        }
-      });
-      y0 = fma(a.dt, c0, y0);
-      y1 = fma(a.dt, c1, y1);
-    }
-  }
-  if (own && valid) {
-    a.fin[j0 * n + p] = y0;
-    a.fin[j1 * n + p] = y1;
-  }
-}
-
 // ------------------------------------------------------------------ adjoint
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
   return v;
 }
+
+}  // namespace gal
+
+#include "stream_pairs.cuh"
+
+namespace gal {
 
 template <class TB>
 __global__ void __launch_bounds__(32) k_stream_particles_adj(StreamDev a, const DevComp* comps) {
@@ -596,9 +412,9 @@ __device__ __forceinline__ void particle_step_of(int64_t q, int64_t& k, int64_t&
   p = q - kk * (kk + 1);
 }
 
-// Hessians at every particle stage point: host + progenitor (0..5) and progenitor alone (6..11).
-template <class TB>
-__global__ void __launch_bounds__(128) k_stream_particle_hess(StreamDev a, const DevComp* comps) {
+// Hessians (host + progenitor) at every particle stage point.
+template <class TB, bool MW>
+__global__ void __launch_bounds__(128) k_stream_particle_hess(StreamDev a, const DevComp* comps, MWParams mwp) {
   __shared__ DevComp s_comps[kAdjMaxComps];
   stage_comps(comps, a.ncomp, s_comps);
   constexpr int S = TB::S;
@@ -610,8 +426,8 @@ __global__ void __launch_bounds__(128) k_stream_particle_hess(StreamDev a, const
   for (int i = 0; i < S; ++i) {
     const double Y[3] = {a.Ys[stage_idx(k, i, 0, p, S, 3)], a.Ys[stage_idx(k, i, 1, p, S, 3)],
                          a.Ys[stage_idx(k, i, 2, p, S, 3)]};
-    double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int c = 0; c < a.ncomp; ++c) comp_hessian(s_comps[c], Y[0], Y[1], Y[2], H);
+    double H[6];
+    host_hessian<MW>(s_comps, a.ncomp, mwp, Y, H);
     const double* Qi = a.Q + (k * S + i) * 3;
     const double d[3] = {Y[0] - Qi[0], Y[1] - Qi[1], Y[2] - Qi[2]};
     const double r2 = fma(d[0], d[0], fma(d[1], d[1], fma(d[2], d[2], TINY)));
@@ -619,103 +435,15 @@ __global__ void __launch_bounds__(128) k_stream_particle_hess(StreamDev a, const
     const double g = a.GMp * is2 * is, gpr = -3.0 * g * is2;
     const double Hp[6] = {fma(gpr * d[0], d[0], g), gpr * d[0] * d[1], gpr * d[0] * d[2],
                           fma(gpr * d[1], d[1], g), gpr * d[1] * d[2], fma(gpr * d[2], d[2], g)};
-    const double Ht[6] = {H[0] + Hp[0], H[1] + Hp[1], H[2] + Hp[2], H[4] + Hp[3], H[5] + Hp[4], H[8] + Hp[5]};
 #pragma unroll
-    for (int e = 0; e < 6; ++e) {
-      a.Hs[stage_idx(k, i, e, p, S, 12)] = Ht[e];
-      a.Hs[stage_idx(k, i, 6 + e, p, S, 12)] = Hp[e];
-    }
-  }
-}
-
-__device__ __forceinline__ void sym_mv(const double* H, const double* v, double* o) {
-  o[0] = fma(H[0], v[0], fma(H[1], v[1], H[2] * v[2]));
-  o[1] = fma(H[1], v[0], fma(H[3], v[1], H[4] * v[2]));
-  o[2] = fma(H[2], v[0], fma(H[4], v[1], H[5] * v[2]));
-}
-
-// Reverse sweep with the stored Hessians: no potential evaluations on the serial chain.
-template <class TB>
-__global__ void __launch_bounds__(32) k_stream_particles_sweep(StreamDev a) {
-  constexpr int S = TB::S;
-  const int lane = threadIdx.x;
-  const int64_t w = blockIdx.x;
-  const int64_t p = w * 32 + lane;
-  const int64_t n = a.np;
-  const bool valid = p < n;
-  const int64_t rp = valid ? (p >> 1) : LLONG_MAX;
-  const int64_t rmin = (w * 32) >> 1;
-  const double dt = a.dt;
-  double lam[6], loss = 0.0;
-#pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    const double d = valid ? a.fin[j * n + p] - a.target[j * n + p] : 0.0;
-    lam[j] = 2.0 * d;
-    loss = fma(d, d, loss);
-  }
-  for (int64_t k = a.n_rel - 1; k >= rmin; --k) {
-    const bool act = valid && k >= rp;
-    double F[S][6];
-    static_for<0, S>([&](auto i) {
-      constexpr int I = decltype(i)::value;
-      constexpr double bi = TB::B[I];
-#pragma unroll
-      for (int j = 0; j < 6; ++j) F[I][j] = dt * bi * lam[j];
-    });
-    double* mw_out = a.mu_warp + (w * a.n_rel + k) * (S * 3);
-    static_for<0, S>([&](auto rr) {
-      constexpr int I = S - 1 - decltype(rr)::value;
-      const double v[3] = {F[I][3], F[I][4], F[I][5]};
-      double Ht[6] = {0, 0, 0, 0, 0, 0}, Hp[6] = {0, 0, 0, 0, 0, 0};
-      if (act) {
-#pragma unroll
-        for (int e = 0; e < 6; ++e) {
-          Ht[e] = a.Hs[stage_idx(k, I, e, p, S, 12)];
-          Hp[e] = a.Hs[stage_idx(k, I, 6 + e, p, S, 12)];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) a.vs[stage_idx(k, I, c, p, S, 3)] = v[c];
-      }
-      double Hv[3], Hpv[3];
-      sym_mv(Ht, v, Hv);
-      sym_mv(Hp, v, Hpv);
-      const double m0 = warp_sum(act ? Hpv[0] : 0.0);
-      const double m1 = warp_sum(act ? Hpv[1] : 0.0);
-      const double m2 = warp_sum(act ? Hpv[2] : 0.0);
-      if (lane == 0) {
-        mw_out[3 * I + 0] = m0;
-        mw_out[3 * I + 1] = m1;
-        mw_out[3 * I + 2] = m2;
-      }
-      const double Yb[6] = {-Hv[0], -Hv[1], -Hv[2], F[I][0], F[I][1], F[I][2]};
-      if (act) {
-#pragma unroll
-        for (int j = 0; j < 6; ++j) lam[j] += Yb[j];
-      }
-      static_for<0, I>([&](auto l) {
-        constexpr int L = decltype(l)::value;
-        constexpr double c = TB::A[I][L];
-        if constexpr (c != 0.0) {
-#pragma unroll
-          for (int j = 0; j < 6; ++j) F[L][j] = fma(dt * c, Yb[j], F[L][j]);
-        }
-      });
-    });
-    if (valid && k == rp) {
-#pragma unroll
-      for (int j = 0; j < 6; ++j) a.lam_rel[j * n + p] = lam[j];
-    }
-  }
-  if (valid) {
-    for (int c = 0; c < 3 * a.ncomp; ++c) a.gp_all[(int64_t)c * a.ncol + p] = 0.0;
-    a.gp_all[(int64_t)(3 * a.ncomp) * a.ncol + p] = loss;
+    for (int e = 0; e < 6; ++e) a.Hs[stage_idx(k, i, e, p, S, 6)] = H[e] + Hp[e];
   }
 }
 
 // Parameter terms -sum d(grad Phi_host . v)/dtheta over all particle stage points,
 // one column of partial sums per block.
-template <class TB>
-__global__ void __launch_bounds__(256) k_stream_particles_pgrad(StreamDev a, const DevComp* comps) {
+template <class TB, bool MW>
+__global__ void __launch_bounds__(256) k_stream_particles_pgrad(StreamDev a, const DevComp* comps, MWParams mwp) {
   __shared__ DevComp s_comps[kAdjMaxComps];
   __shared__ double red[kAdjMaxComps * 3][8];
   stage_comps(comps, a.ncomp, s_comps);
@@ -729,18 +457,31 @@ __global__ void __launch_bounds__(256) k_stream_particles_pgrad(StreamDev a, con
   if (q < nq) {
     int64_t k, p;
     particle_step_of(q, k, p);
+    double gp[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int i = 0; i < S; ++i) {
       const double Y[3] = {a.Ys[stage_idx(k, i, 0, p, S, 3)], a.Ys[stage_idx(k, i, 1, p, S, 3)],
                            a.Ys[stage_idx(k, i, 2, p, S, 3)]};
       const double v[3] = {a.vs[stage_idx(k, i, 0, p, S, 3)], a.vs[stage_idx(k, i, 1, p, S, 3)],
                            a.vs[stage_idx(k, i, 2, p, S, 3)]};
-      for (int c = 0; c < a.ncomp; ++c) {
-        double Hv[3] = {0, 0, 0}, dp[3] = {0, 0, 0};
-        comp_vjp(s_comps[c], Y, v, Hv, dp);
-        acc[3 * c + 0] -= dp[0];
-        acc[3 * c + 1] -= dp[1];
-        acc[3 * c + 2] -= dp[2];
+      if constexpr (MW) {
+        double w[7], g[3], Hv[3];
+        mw_stage(mwp, Y, w, g);
+        mw_stage_vjp(mwp, Y, w, v, Hv, gp);
+      } else {
+        for (int c = 0; c < a.ncomp; ++c) {
+          double Hv[3] = {0, 0, 0}, dp[3] = {0, 0, 0};
+          comp_vjp(s_comps[c], Y, v, Hv, dp);
+          acc[3 * c + 0] -= dp[0];
+          acc[3 * c + 1] -= dp[1];
+          acc[3 * c + 2] -= dp[2];
+        }
       }
+    }
+    if constexpr (MW) {
+      double out[12];
+      mw_param_grads(mwp, s_comps, gp, out);
+#pragma unroll
+      for (int c = 0; c < 12; ++c) acc[c] = -out[c];
     }
   }
   // warp sums, then the block's eight warps in order
@@ -1249,7 +990,8 @@ __global__ void __launch_bounds__(128) k_stream_release_adj(StreamDev a, const D
 // velocity cotangent v of every stage; the parameter gradient
 // -sum d(grad Phi . v)/dtheta over all stage points is again parallel
 // (k_stream_prog_pgrad).
-__global__ void __launch_bounds__(128) k_stream_prog_hess(StreamDev a, const DevComp* comps, int S) {
+template <bool MW>
+__global__ void __launch_bounds__(128) k_stream_prog_hess(StreamDev a, const DevComp* comps, MWParams mwp, int S) {
   __shared__ DevComp s_comps[kAdjMaxComps];
   stage_comps(comps, a.ncomp, s_comps);
   const int64_t npts = 2 * a.n_rel * S;
@@ -1257,80 +999,7 @@ __global__ void __launch_bounds__(128) k_stream_prog_hess(StreamDev a, const Dev
   if (p >= npts) return;
   const int64_t per = a.n_rel * S;
   const double* Y = (p < per ? a.Q + 3 * p : a.Qb + 3 * (p - per));
-  double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int c = 0; c < a.ncomp; ++c) comp_hessian(s_comps[c], Y[0], Y[1], Y[2], H);
-  double* o = a.Hst + 6 * p;
-  o[0] = H[0];
-  o[1] = H[1];
-  o[2] = H[2];
-  o[3] = H[4];
-  o[4] = H[5];
-  o[5] = H[8];
-}
-
-// One track of the reverse recurrence (track 0: forwards, hs = +dt, with the
-// particles' cotangents mu on the stage positions and the release-map
-// cotangents nu on the grid states; track 1: backwards, hs = -dt). Lane j < 6
-// owns component j of lambda and of every stage cotangent Fbar_i.
-template <class TB>
-__device__ __forceinline__ void prog_sweep_track(const StreamDev& a, int track, double hs, double& lam, int lane) {
-  constexpr int S = TB::S;
-  const bool mine = lane < 6;
-  const int hrow = lane < 3 ? lane : 0;
-  const int h0 = hrow == 0 ? 0 : (hrow == 1 ? 1 : 2);
-  const int h1 = hrow == 0 ? 1 : (hrow == 1 ? 3 : 4);
-  const int h2 = hrow == 0 ? 2 : (hrow == 1 ? 4 : 5);
-  const int src = (lane >= 3 && lane < 6) ? lane - 3 : lane;
-  for (int64_t k = a.n_rel - 1; k >= 0; --k) {
-    const int64_t base = (int64_t)track * a.n_rel * S + k * S;  // stage-point index of (k, 0)
-    double Hr[S][3], Mu[S];
-    // all of this step's inputs in flight together
-    static_for<0, S>([&](auto i) {
-      constexpr int I = decltype(i)::value;
-      const double* Hp = a.Hst + 6 * (base + I);
-      Hr[I][0] = lane < 3 ? Hp[h0] : 0.0;
-      Hr[I][1] = lane < 3 ? Hp[h1] : 0.0;
-      Hr[I][2] = lane < 3 ? Hp[h2] : 0.0;
-      Mu[I] = (track == 0 && lane < 3) ? a.mu[(k * S + I) * 3 + lane] : 0.0;
-    });
-    const double nu = (track == 0 && mine) ? a.nu[6 * k + lane] : 0.0;
-    double Fb[S];
-    static_for<0, S>([&](auto i) {
-      constexpr int I = decltype(i)::value;
-      constexpr double bi = TB::B[I];
-      Fb[I] = hs * bi * lam;
-    });
-    static_for<0, S>([&](auto rr) {
-      constexpr int I = S - 1 - decltype(rr)::value;
-      const double f = Fb[I];
-      const double v0 = __shfl_sync(0xffffffffu, f, 3);
-      const double v1 = __shfl_sync(0xffffffffu, f, 4);
-      const double v2 = __shfl_sync(0xffffffffu, f, 5);
-      const double pos = __shfl_sync(0xffffffffu, f, src);
-      if (lane >= 3 && mine) a.vst[3 * (base + I) + (lane - 3)] = f;
-      double Yb;
-      if (lane < 3)
-        Yb = Mu[I] - fma(Hr[I][0], v0, fma(Hr[I][1], v1, Hr[I][2] * v2));
-      else
-        Yb = mine ? pos : 0.0;
-      lam += Yb;
-      static_for<0, I>([&](auto l) {
-        constexpr int L = decltype(l)::value;
-        constexpr double c = TB::A[I][L];
-        if constexpr (c != 0.0) Fb[L] = fma(hs * c, Yb, Fb[L]);
-      });
-    });
-    lam += nu;
-  }
-}
-
-template <class TB>
-__global__ void __launch_bounds__(32) k_stream_prog_sweep(StreamDev a) {
-  const int lane = threadIdx.x;
-  double lam = 0.0;
-  prog_sweep_track<TB>(a, 0, a.dt, lam, lane);
-  prog_sweep_track<TB>(a, 1, -a.dt, lam, lane);
-  if (a.grad_w_now && lane < 6) a.grad_w_now[lane] = lam;
+  host_hessian<MW>(s_comps, a.ncomp, mwp, Y, a.Hst + 6 * p);
 }
 
 __global__ void __launch_bounds__(128) k_stream_prog_pgrad(StreamDev a, const DevComp* comps, int S) {
@@ -1408,14 +1077,14 @@ static StreamLayout stream_layout(int ncomp, const gal_stream_config& c, bool gr
     L.vst = take(d * 3 * 2 * L.S * nr);
     if (stored) {
       L.Ys = take(d * 3 * L.S * (size_t)nq);
-      L.Hs = take(d * 12 * L.S * (size_t)nq);
+      L.Hs = take(d * 6 * L.S * (size_t)nq);
       L.vs = take(d * 3 * L.S * (size_t)nq);
     } else {
       L.ckpt = take(d * 6 * L.nseg * L.np);
       L.seg = take(d * 6 * (size_t)K * L.np);
     }
     L.lam_rel = take(d * 6 * L.np);
-    L.mu_warp = take(d * 3 * L.S * nr * L.nwarps);
+    if (!stored) L.mu_warp = take(d * 3 * L.S * nr * L.nwarps);
     L.mu = take(d * 3 * L.S * nr);
     L.nu = take(d * 6 * nr);
     L.gp_all = take(d * (3 * (size_t)ncomp + 1) * L.ncol);
@@ -1487,7 +1156,7 @@ static StreamDev stream_args(const gal_potential* pot, const gal_stream_config* 
       a.seg = at(L.seg);
     }
     a.lam_rel = at(L.lam_rel);
-    a.mu_warp = at(L.mu_warp);
+    if (c->k_ckpt != 0) a.mu_warp = at(L.mu_warp);
     a.mu = at(L.mu);
     a.nu = at(L.nu);
     a.gp_all = at(L.gp_all);
@@ -1498,30 +1167,29 @@ static StreamDev stream_args(const gal_potential* pot, const gal_stream_config* 
 template <class TB>
 static cudaError_t stream_forward(const StreamDev& a, const gal_potential* pot, cudaStream_t s) {
   const DevComp* comps = pot->d_comps;
-  if (pot->is_mw)
-    k_stream_progenitor_mw<TB><<<1, 128, 0, s>>>(a, pot->mw);
-  else
-    k_stream_progenitor_team<TB><<<1, 128, 0, s>>>(a, comps);
+  if (pot->is_mw) k_stream_progenitor_mw<TB><<<1, 128, 0, s>>>(a, pot->mw);
+  else k_stream_progenitor_team<TB><<<1, 128, 0, s>>>(a, comps);
   k_stream_release<<<(unsigned)((a.n_rel + 127) / 128), 128, 0, s>>>(a, comps);
-  k_stream_particles_team<TB><<<(unsigned)((a.np + 31) / 32), 128, 0, s>>>(a, comps);
+  k_stream_particles_team<TB><<<(unsigned)((a.np + 15) / 16), 128, 0, s>>>(a, comps);
   return cudaGetLastError();
 }
 
-template <class TB>
-static cudaError_t stream_backward(const StreamDev& a, const DevComp* comps, cudaStream_t s) {
+template <class TB, bool MW>
+static cudaError_t stream_backward(const StreamDev& a, const DevComp* comps, const MWParams& mwp, cudaStream_t s) {
+  const int S3 = 3 * TB::S;
   if (a.Ys) {
     const int64_t nq = a.n_rel * (a.n_rel + 1);
-    k_stream_particle_hess<TB><<<(unsigned)((nq + 127) / 128), 128, 0, s>>>(a, comps);
-    k_stream_particles_sweep<TB><<<(unsigned)a.nwarps, 32, 0, s>>>(a);
-    k_stream_particles_pgrad<TB><<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(a, comps);
+    k_stream_particle_hess<TB, MW><<<(unsigned)((nq + 127) / 128), 128, 0, s>>>(a, comps, mwp);
+    k_stream_particles_sweep<TB><<<(unsigned)((a.np + kSweepParticles - 1) / kSweepParticles), 32, 0, s>>>(a);
+    k_stream_particles_pgrad<TB, MW><<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(a, comps, mwp);
+    k_stream_mu<<<(unsigned)((a.n_rel * TB::S + 3) / 4), 128, 0, s>>>(a, TB::S);
   } else {
     k_stream_particles_adj<TB><<<(unsigned)a.nwarps, 32, 0, s>>>(a, comps);
+    k_stream_mu_reduce<<<(unsigned)((a.n_rel * S3 + 255) / 256), 256, 0, s>>>(a, S3);
   }
-  const int S3 = 3 * TB::S;
-  k_stream_mu_reduce<<<(unsigned)((a.n_rel * S3 + 255) / 256), 256, 0, s>>>(a, S3);
   k_stream_release_adj<<<(unsigned)((a.n_rel + 127) / 128), 128, 0, s>>>(a, comps);
   const int64_t npts = 2 * a.n_rel * TB::S;
-  k_stream_prog_hess<<<(unsigned)((npts + 127) / 128), 128, 0, s>>>(a, comps, TB::S);
+  k_stream_prog_hess<MW><<<(unsigned)((npts + 127) / 128), 128, 0, s>>>(a, comps, mwp, TB::S);
   k_stream_prog_sweep<TB><<<1, 32, 0, s>>>(a);
   k_stream_prog_pgrad<<<(unsigned)((npts + 127) / 128), 128, 0, s>>>(a, comps, TB::S);
   return cudaGetLastError();
@@ -1608,7 +1276,8 @@ gal_status gal_stream_grad(const gal_potential* pot, const gal_stream_config* cf
   cudaError_t e = dispatch(cfg->method, [&](auto tb) {
     cudaError_t e1 = stream_forward<decltype(tb)>(a, pot, s);
     if (e1 != cudaSuccess) return e1;
-    return stream_backward<decltype(tb)>(a, pot->d_comps, s);
+    if (pot->is_mw) return stream_backward<decltype(tb), true>(a, pot->d_comps, pot->mw, s);
+    return stream_backward<decltype(tb), false>(a, pot->d_comps, pot->mw, s);
   });
   if (e != cudaSuccess) return cuda_fail(e, "stream gradient kernels");
   double* red = reinterpret_cast<double*>(ws + L.red);
