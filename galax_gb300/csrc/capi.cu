@@ -101,6 +101,80 @@ static MWParams mw_params(const gal_component* c, double G) {
   return p;
 }
 
+// The table's Plummer spheres in fixed point (fixed_plummer.cuh), where their
+// scales fit; p->fixed.n = 0 otherwise. Allocates on the first call for a handle
+// (the number of components never changes).
+static cudaError_t build_fixed(gal_potential* p) {
+  p->fixed = FixedTable{};
+  std::vector<int32_t> at, other;
+  double reach = 0.0;
+  for (int i = 0; i < p->n; ++i) {
+    const gal_component& c = p->comps[i];
+    if (c.kind != GAL_PLUMMER) {
+      other.push_back(i);
+      continue;
+    }
+    at.push_back(i);
+    for (double v : c.origin) reach = std::fmax(reach, std::fabs(v));
+    reach = std::fmax(reach, c.l1);
+  }
+  if ((int)at.size() < kWarpMinComponents || !(reach > 0.0)) return cudaSuccess;
+  int top = 0;
+  std::frexp(reach, &top);       // reach <= 2^top
+  const int xtop = top + 2;      // positions up to 2^xtop: offsets below 2^(xtop + 1)
+  const int s = 60 - 1 - xtop;   // ... and below 2^60 in units of 2^-s
+  if (std::abs(s) > 900) return cudaSuccess;
+  std::vector<FixedPlummer> h(at.size());
+  for (size_t i = 0; i < at.size(); ++i) {
+    const gal_component& c = p->comps[at[i]];
+    FixedPlummer& f = h[i];
+    f = FixedPlummer{};
+    for (int j = 0; j < 3; ++j) f.c[j] = std::llrint(std::ldexp(c.origin[j], s));
+    const double Gm = p->G * c.m;
+    int e = 0;
+    f.gm = (uint64_t)std::ldexp(std::frexp(std::fabs(Gm), &e), 64);
+    f.sign = Gm < 0.0 ? 0x80000000u : 0u;
+    f.e0 = (e - 64) - 178 + 2 * s;
+    if (f.gm != 0 && (f.e0 < -1000 || f.e0 > 800)) return cudaSuccess;  // the result's exponent stays normal
+    if (c.l1 > 0.0) {
+      const double b = std::ldexp(c.l1, s);
+      f.bhi = (uint32_t)((uint64_t)b >> 32);
+      int eb = 0;
+      const double m = std::frexp(b, &eb);  // b = m 2^eb; 2^kb b in [2^60, 2^61)
+      f.kb = 61 - eb;
+      if (f.kb > 1000) return cudaSuccess;
+      const uint64_t n = (uint64_t)std::ldexp(m, 53);  // exact; b2 = (n 2^8)^2 / 2^60 = n^2 / 2^44
+      const uint64_t hi = n >> 32, lo = n & 0xffffffffu;
+      f.b2 = (hi * hi << 20) + ((hi * lo) >> 11) + ((lo * lo) >> 44);
+    }
+  }
+  at.insert(at.end(), other.begin(), other.end());
+  const size_t records = sizeof(FixedPlummer) * h.size();
+  cudaError_t e = cudaSuccess;
+  if (!p->d_fixed) e = cudaMalloc(&p->d_fixed, sizeof(FixedPlummer) * (size_t)p->n + sizeof(int32_t) * (size_t)p->n);
+  if (e != cudaSuccess) {
+    p->d_fixed = nullptr;
+    return e;
+  }
+  char* base = static_cast<char*>(p->d_fixed);
+  e = cudaMemcpy(base, h.data(), records, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(base + records, at.data(), sizeof(int32_t) * at.size(), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return e;
+  p->fixed.f = reinterpret_cast<const FixedPlummer*>(base);
+  p->fixed.at = reinterpret_cast<const int32_t*>(base + records);
+  p->fixed.n = (int)h.size();
+  p->fixed.nother = (int)other.size();
+  p->fixed.s = s;
+  p->fixed.scale = std::ldexp(1.0, s);
+  p->fixed.xmax = std::ldexp(1.0, xtop);
+  gal_component four[4];
+  p->fixed_mw = other.size() == 4;
+  for (size_t i = 0; i < other.size() && i < 4; ++i) four[i] = p->comps[other[i]];
+  p->fixed_mw = p->fixed_mw && milky_way_shape(four, 4);
+  p->fixed_mwp = p->fixed_mw ? mw_params(four, p->G) : MWParams{};
+  return cudaSuccess;
+}
+
 static gal_status validate_components(const gal_component* comps, int32_t n) {
   if (!comps || n < 1) return fail(GAL_ERR_INVALID_ARGUMENT, "need at least one component");
   if (n > GAL_MAX_COMPONENTS) return fail(GAL_ERR_TOO_LARGE, "too many components (max GAL_MAX_COMPONENTS)");
@@ -411,6 +485,12 @@ gal_status gal_potential_create(const gal_component* comps, int32_t n, double G,
       cudaFree(p->d_comps);
       return cuda_fail(e, "cudaMemcpy(component table)");
     }
+    e = build_fixed(p);
+    if (e != cudaSuccess) {
+      cudaFree(p->d_comps);
+      cudaFree(p->d_fixed);
+      return cuda_fail(e, "fixed-point table");
+    }
     *out = holder.release();
     return GAL_OK;
   });
@@ -419,6 +499,10 @@ gal_status gal_potential_create(const gal_component* comps, int32_t n, double G,
 gal_status gal_potential_destroy(gal_potential* p) {
   if (!p) return GAL_OK;
   cudaError_t e = cudaFree(p->d_comps);
+  if (p->d_fixed) {
+    const cudaError_t e1 = cudaFree(p->d_fixed);
+    if (e == cudaSuccess) e = e1;
+  }
   if (p->d_lin) {
     const cudaError_t e2 = cudaFree(p->d_lin);
     if (e == cudaSuccess) e = e2;
@@ -490,6 +574,8 @@ gal_status gal_potential_update(gal_potential* p, const gal_component* comps, in
     p->comps.assign(comps, comps + n);
     p->is_mw = !p->d_lin && milky_way_shape(comps, n);
     p->mw = milky_way_shape(comps, n) ? mw_params(comps, p->G) : MWParams{};
+    e = build_fixed(p);
+    if (e != cudaSuccess) return cuda_fail(e, "fixed-point table");
     if (p->d_lin) {  // new values at t = 0, same slopes
       std::vector<DevLinear> L(n);
       e = cudaMemcpy(L.data(), p->d_lin, sizeof(DevLinear) * n, cudaMemcpyDeviceToHost);
@@ -661,6 +747,9 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   a.order = order;
   a.n = n;
   a.lin = p->d_lin;
+  a.fixed = p->fixed;
+  a.fixed_mw = p->fixed_mw ? 1 : 0;
+  a.fixed_mwp = p->fixed_mwp;
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = static_cast<char*>(workspace);
   a.queue = reinterpret_cast<unsigned long long*>(ws);
@@ -670,11 +759,11 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   a.queue_len = nullptr;
   const LaunchShape shape = launch_shape(cfg->method, cfg->adaptive);
   // Dopri8 saves as one parallel pass afterwards (put_deferred_save) when the
-  // workspace has an entry per save. Not for one warp per orbit, whose component
+  // workspace has an entry per save. Not for several lanes per orbit, whose component
   // sums a per-save thread would not repeat bit for bit, and not for saves in
   // host memory, which would cross the bus three times.
   if (cfg->method == 8 && total > 0 && workspace_bytes >= align256(need) + sizeof(double) * (size_t)total &&
-      (p->is_mw || !dopri8_warp_per_orbit(shape, n, p->n))) {
+      (p->is_mw || !dopri8_inline_saves(a, shape, p->n))) {
     cudaPointerAttributes attr{};
     if (cudaPointerGetAttributes(&attr, out) != cudaSuccess) {
       cudaGetLastError();

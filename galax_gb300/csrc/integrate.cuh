@@ -29,6 +29,7 @@
 
 #include <cstdint>
 
+#include "fixed_plummer.cuh"
 #include "potentials.cuh"
 #include "tableaux.cuh"
 
@@ -112,6 +113,9 @@ struct IntegrateArgs {
   int64_t n;
   unsigned long long* queue;  // work-queue counter (scratch)
   const DevLinear* lin;       // time-dependent component parameters (table kernel), or NULL
+  FixedTable fixed;           // the table's Plummer spheres in fixed point (n = 0: not used)
+  int32_t fixed_mw;           // its other components are the Milky Way's four
+  MWParams fixed_mwp;
   // two-phase schedule: phase 0 parks every orbit once it has covered split_frac
   // of its span; phase 1 resumes the parked orbits from `resume` in `order`
   int32_t phase;
@@ -416,9 +420,9 @@ __device__ __forceinline__ void first_step(const IntegrateArgs& a, OrbitState& s
 // does not queue up on a few FP64 pipes. Later positions are dequeued
 // atomically after the gridDim.x * blockDim.x striped ones.
 //
-// With LANES = 32 a whole warp owns one orbit (warp-per-orbit mode, for
-// composites with many components): the positions are handed out per warp,
-// and lane 0 takes the next one from the queue for the warp.
+// With several lanes per orbit (composites with many components; a whole warp
+// with LANES = 32) the positions are handed out per group of lanes, and its first
+// lane takes the next one from the queue for the group.
 //
 // Blocks: the `count` blocks of a launch that share one arrangement, of which
 // this is number `index`, and their first queue position (all blocks and 0, but
@@ -429,21 +433,30 @@ struct Blocks {
 };
 __device__ __forceinline__ Blocks all_blocks() { return Blocks{gridDim.x, blockIdx.x, 0}; }
 
-template <int LANES>
-__device__ __forceinline__ unsigned long long first_position(const Blocks& g) {
+__device__ __forceinline__ unsigned long long first_position(const Blocks& g, int lanes) {
   const unsigned long long W = blockDim.x >> 5, w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if constexpr (LANES == 32) return w * g.count + g.index;
+  if (lanes > 1) return (unsigned long long)(threadIdx.x / lanes) * g.count + g.index;
   return (l * W + w) * g.count + g.index;
 }
 
-template <int LANES>
-__device__ __forceinline__ unsigned long long next_position(unsigned long long* queue) {
-  if constexpr (LANES == 32) {
+__device__ __forceinline__ unsigned group_mask(int lanes) {
+  return lanes >= 32 ? 0xffffffffu : ((1u << lanes) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(lanes - 1));
+}
+
+__device__ __forceinline__ unsigned long long next_position(unsigned long long* queue, int lanes) {
+  if (lanes > 1) {
     unsigned long long k = 0;
-    if ((threadIdx.x & 31) == 0) k = atomicAdd(queue, 1ULL);
-    return __shfl_sync(0xffffffffu, k, 0);
+    if ((threadIdx.x & (lanes - 1)) == 0) k = atomicAdd(queue, 1ULL);
+    return __shfl_sync(group_mask(lanes), k, (threadIdx.x & 31) & ~(lanes - 1));
   }
   return atomicAdd(queue, 1ULL);
+}
+
+// Lanes per orbit: LANES, or with LANES = 0 a power of two that the model holds.
+template <int LANES, class Pot>
+__device__ __forceinline__ int lanes_of(const Pot& pot) {
+  if constexpr (LANES == 0) return pot.lanes;
+  else return LANES;
 }
 
 // Returns false when the queue is empty.
@@ -451,15 +464,16 @@ template <class TB, class Pot, int LANES = 1>
 __device__ __forceinline__ bool start_orbit(const IntegrateArgs& a, const Pot& pot, const Blocks& g, OrbitState& s,
                                             bool& first) {
   const unsigned long long qlen = a.queue_len ? *a.queue_len : (unsigned long long)a.n;
-  const unsigned long long striped = (unsigned long long)g.count * (blockDim.x / LANES);
+  const int lanes = lanes_of<LANES>(pot);
+  const unsigned long long striped = (unsigned long long)g.count * (blockDim.x / lanes);
   const unsigned long long base = (unsigned long long)g.base;
   while (true) {
     unsigned long long k;
     if (first) {
       first = false;
-      k = base + first_position<LANES>(g);
+      k = base + first_position(g, lanes);
     } else {
-      k = base + striped + next_position<LANES>(a.queue);
+      k = base + striped + next_position(a.queue, lanes);
     }
     if (k >= qlen) return false;
     const int64_t o = a.order ? (int64_t)a.order[k] : (int64_t)k;
@@ -615,10 +629,11 @@ __device__ __forceinline__ double clip_to_end(double tprev, double tnext, double
   return tnext;
 }
 
-// LANES = 1: one thread per orbit. LANES = 32: one warp per orbit; Pot must
-// then give every lane of the warp the bitwise-same gradient (WarpTablePot), so
-// the 32 lanes run the orbit's steps in lockstep on identical values and their
-// identical stores of saves, status and steps coincide.
+// LANES = 1: one thread per orbit. LANES = 32: one warp per orbit; LANES = 0: the
+// model's number of lanes. With several lanes Pot must give each of them the
+// bitwise-same gradient (WarpTablePot, FixedTablePot), so that they run the
+// orbit's steps in lockstep on identical values and their identical stores of
+// saves, status and steps coincide.
 template <class TB, class Pot, int LANES = 1>
 __device__ void integrate_loop(const IntegrateArgs& a, const Pot& pot, const Blocks& g = all_blocks()) {
   OrbitState s;

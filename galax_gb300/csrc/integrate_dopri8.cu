@@ -15,8 +15,8 @@ cudaError_t launch_deferred_saves8(const IntegrateArgs& a, bool mw, const MWPara
   return launch_deferred_saves<Dopri8>(a, mw, p, comps, ncomp, stream);
 }
 
-bool dopri8_warp_per_orbit(const LaunchShape& shape, int64_t n, int ncomp) {
-  return use_warp_per_orbit(shape, n, ncomp);
+bool dopri8_inline_saves(const IntegrateArgs& a, const LaunchShape& shape, int ncomp) {
+  return use_fixed(a, shape) || use_warp_per_orbit(shape, a.n, ncomp);
 }
 
 cudaError_t launch_integrate_team8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,

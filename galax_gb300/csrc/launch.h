@@ -39,8 +39,8 @@ cudaError_t launch_integrate_mixed8(const IntegrateArgs& a, const MWParams& p, c
 // Dopri8 saves left to a.defer (put_deferred_save), after the integration on the same stream.
 cudaError_t launch_deferred_saves8(const IntegrateArgs& a, bool mw, const MWParams& p, const DevComp* comps, int ncomp,
                                    cudaStream_t stream);
-// Whether such a batch runs one warp per orbit, whose sums have another order than one thread's.
-bool dopri8_warp_per_orbit(const LaunchShape& shape, int64_t n, int ncomp);
+// Whether a table's batch runs several lanes per orbit, whose sums one thread per save would not repeat.
+bool dopri8_inline_saves(const IntegrateArgs& a, const LaunchShape& shape, int ncomp);
 // Batches of at most this many orbits per SM run on teams alone.
 constexpr int kTeamOrbitsPerSm = 4 * kTeamLanes;
 constexpr size_t kExclusiveSmem = 120 * 1024;
