@@ -1,13 +1,13 @@
 // Orbit integration with the learned surrogate: analytic FP64 part + MLP part.
 //
-// Dopri5 with a constant step over a batch of orbits, stepped at batch level:
-// per stage one FP64 kernel forms the stage state Y = y + h sum_l a_il F_l,
-// writes F_i = (Y_v, -grad Phi_analytic(Y_q)) and the stage positions, then the
-// tensor-core MLP kernel adds -grad Phi_MLP(Y_q) into F_i. The seventh stage is
-// evaluated at y_{n+1} (FSAL), so it becomes the next step's first slope in
-// place. One step (12 kernels) is captured once as a CUDA graph and replayed.
-// The analytic part is any gal_potential (the Milky Way model runs its
-// specialised gradient).
+// Dopri5 with a constant step over a batch of orbits, stepped at batch level. Per
+// stage one kernel forms the stage state Y = y + h sum_l a_il F_l, its positions
+// and the near field there; the tensor-core MLP kernel and the FP64 kernel of the
+// analytic part then evaluate the two terms of F_i = (Y_v, -grad Phi(Y_q)) side by
+// side. The seventh stage is evaluated at y_{n+1} (FSAL), so it becomes the next
+// step's first slope in place. One step is captured once as a CUDA graph and
+// replayed. Without a network, one kernel per stage does it all. The analytic part
+// is any gal_potential (the Milky Way model runs its specialised gradient).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -84,27 +84,164 @@ __global__ void __launch_bounds__(256) k_slope0(Pot pot, const double* __restric
   }
 }
 
+// With a network, a stage is three kernels. k_state forms the stage state from the
+// slopes and sums the near field there; then the network's term (tensor cores) and
+// the analytic one (FP64) are evaluated side by side, the one into the slope's own
+// place, the other into A [3][n], onto the near field; the next k_state adds the
+// two, A first, and leaves the sum as the slope. The network kernel holds each SM's
+// shared memory, and with it all but a few KB of L1, and all but 11,776 of its
+// registers; the analytic kernel's one block of two warps per SM fits into these
+// and passes under the network's time. (The near field does not: its lists need the
+// L1 and many warps, 54 ms for the steps below.) 131,072 orbits, 20 steps, with a
+// near field of 512 spheres: 23.7 -> 20.9 ms; without: 18.8 -> 16.6 ms; 500 orbits: 8.6
+// -> 5.6 ms.
+//
+// Stage I of a step from (y, F): as k_stage, without the gradient; P is the slot of
+// the previous stage, whose two terms are still apart.
+template <int I, class Pot>
+__global__ void __launch_bounds__(256) k_state(Pot pot, double* __restrict__ y, double* __restrict__ F,
+                                               double* __restrict__ Yq, double* __restrict__ A, double hs, int64_t n) {
+  constexpr int P = I - 1;
+  constexpr int slot = (I == Dopri5::S - 1) ? 0 : I;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t first = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); first < n; first += stride) {
+    const int64_t own = first + (threadIdx.x & 31);
+    const bool valid = own < n;
+    const int64_t i = valid ? own : n - 1;  // the last warp's spare lanes follow its last orbit and write nothing
+    double Y[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      double last = F[((int64_t)P * 6 + j) * n + i];
+      if (j >= 3) last = A[(j - 3) * n + i] + last;
+      double acc = 0.0;
+      bool first = true;
+      static_for<0, I>([&](auto l) {
+        constexpr int L = decltype(l)::value;
+        constexpr double c = Dopri5::A[I][L];
+        if constexpr (c != 0.0) {
+          const double f = L == P ? last : F[((int64_t)L * 6 + j) * n + i];
+          acc = first ? c * f : fma(c, f, acc);
+          first = false;
+        }
+      });
+      Y[j] = fma(hs, acc, y[(int64_t)j * n + i]);
+    }
+    float near[3];
+    const bool has_near = near_grad(pot, Y[0], Y[1], Y[2], near);
+    if (!valid) continue;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int64_t a = ((int64_t)P * 6 + 3 + j) * n + i;
+      F[a] = A[j * n + i] + F[a];  // the slope itself, for the later stages
+      F[((int64_t)slot * 6 + j) * n + i] = Y[3 + j];
+      Yq[(int64_t)j * n + i] = Y[j];
+    }
+    if (has_near) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) A[(int64_t)j * n + i] = (double)near[j];
+    }
+    if constexpr (I == Dopri5::S - 1) {
+#pragma unroll
+      for (int j = 0; j < 6; ++j) y[(int64_t)j * n + i] = Y[j];  // y_{n+1} = Y_7 (a_7 = b)
+    }
+  }
+}
+
+// The first step's first slope: its position, velocity part and near field.
 template <class Pot>
-static cudaError_t launch_step(const Pot& pot, double* y, double* F, double* Yq, double hs, int64_t n,
-                               const gal_mlp* mlp, cudaStream_t s, unsigned grid) {
-  auto mlp_add = [&](double* Fslot) -> cudaError_t {
-    if (!mlp) return cudaSuccess;
-    return gal_mlp_eval(mlp, Yq, n, Fslot + 3 * n, 1, -1.0, nullptr, s) == GAL_OK ? cudaSuccess
-                                                                                    : cudaErrorLaunchFailure;
-  };
-  cudaError_t e;
-  k_stage<1><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
-  if ((e = mlp_add(F + 1 * 6 * n)) != cudaSuccess) return e;
-  k_stage<2><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
-  if ((e = mlp_add(F + 2 * 6 * n)) != cudaSuccess) return e;
-  k_stage<3><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
-  if ((e = mlp_add(F + 3 * 6 * n)) != cudaSuccess) return e;
-  k_stage<4><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
-  if ((e = mlp_add(F + 4 * 6 * n)) != cudaSuccess) return e;
-  k_stage<5><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
-  if ((e = mlp_add(F + 5 * 6 * n)) != cudaSuccess) return e;
-  k_stage<6><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);  // FSAL: slot 0 and y_{n+1}
-  if ((e = mlp_add(F)) != cudaSuccess) return e;
+__global__ void __launch_bounds__(256) k_state0(Pot pot, const double* __restrict__ y, double* __restrict__ F,
+                                                double* __restrict__ Yq, double* __restrict__ A, int64_t n) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t first = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); first < n; first += stride) {
+    const int64_t own = first + (threadIdx.x & 31);
+    const int64_t i = own < n ? own : n - 1;
+    const double x[3] = {y[i], y[n + i], y[2 * n + i]};
+    float near[3];
+    const bool has_near = near_grad(pot, x[0], x[1], x[2], near);
+    if (own >= n) continue;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      F[(int64_t)j * n + i] = y[(int64_t)(3 + j) * n + i];
+      Yq[(int64_t)j * n + i] = x[j];
+      if (has_near) A[(int64_t)j * n + i] = (double)near[j];
+    }
+  }
+}
+
+// Two warps, one per sub-partition that has room beside the network's ten (three on
+// each of two sub-partitions, two on the others): at most 168 registers.
+constexpr int kAnalyticBlock = 64;
+
+// A: -(analytic gradient + the near field that k_state left there).
+template <class Pot>
+__global__ void __launch_bounds__(kAnalyticBlock, 6) k_analytic(Pot pot, const double* __restrict__ Yq,
+                                                                double* __restrict__ A, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double g[3];
+    const bool has_near = far_grad(pot, Yq[i], Yq[n + i], Yq[2 * n + i], g);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      if (has_near) g[j] += A[j * n + i];
+      A[j * n + i] = -g[j];
+    }
+  }
+}
+
+// The side stream of the analytic term, and the events that order it.
+struct Side {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaError_t create() {
+    cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+    return e;
+  }
+  // queued work still completes
+  ~Side() {
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (stream) cudaStreamDestroy(stream);
+  }
+};
+
+// Both terms at Yq: the network's into slot[3 n ..), the analytic one into A.
+template <class Pot>
+static cudaError_t launch_terms(const Pot& pot, const double* Yq, double* slot, double* A, int64_t n,
+                                const gal_mlp* mlp, cudaStream_t s, Side& side) {
+  cudaError_t e = cudaEventRecord(side.fork, s);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(side.stream, side.fork, 0);
+  if (e != cudaSuccess) return e;
+  // whatever fails from here on, the caller's stream waits for what was queued on the side
+  const bool mlp_ok = gal_mlp_eval(mlp, Yq, n, slot + 3 * n, 0, -1.0, nullptr, s) == GAL_OK;
+  const int64_t blocks = (n + kAnalyticBlock - 1) / kAnalyticBlock, sms = device_sm_count();
+  k_analytic<<<(unsigned)(blocks < sms ? blocks : sms), kAnalyticBlock, 0, side.stream>>>(pot, Yq, A, n);
+  e = cudaGetLastError();
+  const cudaError_t e1 = cudaEventRecord(side.join, side.stream);
+  const cudaError_t e2 = e1 == cudaSuccess ? cudaStreamWaitEvent(s, side.join, 0) : e1;
+  if (!mlp_ok) return cudaErrorLaunchFailure;
+  return e != cudaSuccess ? e : e2;
+}
+
+template <class Pot>
+static cudaError_t launch_step_mlp(const Pot& pot, double* y, double* F, double* Yq, double* A, double hs, int64_t n,
+                                   const gal_mlp* mlp, cudaStream_t s, Side& side, unsigned grid) {
+  cudaError_t e = cudaSuccess;
+  static_for<1, Dopri5::S>([&](auto i) {
+    constexpr int I = decltype(i)::value;
+    if (e != cudaSuccess) return;
+    k_state<I><<<grid, 256, 0, s>>>(pot, y, F, Yq, A, hs, n);
+    e = launch_terms(pot, Yq, F + (int64_t)(I == Dopri5::S - 1 ? 0 : I) * 6 * n, A, n, mlp, s, side);
+  });
+  return e;
+}
+
+template <class Pot>
+static cudaError_t launch_step(const Pot& pot, double* y, double* F, double* Yq, double hs, int64_t n, cudaStream_t s,
+                               unsigned grid) {
+  static_for<1, Dopri5::S>([&](auto i) {
+    k_stage<decltype(i)::value><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
+  });
   return cudaGetLastError();
 }
 
@@ -118,7 +255,7 @@ extern "C" {
 
 gal_status gal_surrogate_workspace_size(int64_t n, size_t* bytes) {
   if (!bytes || n < 0) return fail(GAL_ERR_INVALID_ARGUMENT, "bad workspace query");
-  *bytes = align256(sizeof(double) * 7 * 6 * (size_t)n) + align256(sizeof(double) * 3 * (size_t)n);
+  *bytes = align256(sizeof(double) * 7 * 6 * (size_t)n) + 2 * align256(sizeof(double) * 3 * (size_t)n);
   return GAL_OK;
 }
 
@@ -134,7 +271,13 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   if (!workspace || workspace_bytes < need) return fail(GAL_ERR_WORKSPACE, "workspace too small");
   double* F = static_cast<double*>(workspace);
   double* Yq = reinterpret_cast<double*>(static_cast<char*>(workspace) + align256(sizeof(double) * 7 * 6 * (size_t)n));
+  double* A = reinterpret_cast<double*>(reinterpret_cast<char*>(Yq) + align256(sizeof(double) * 3 * (size_t)n));
   cudaStream_t caller = (cudaStream_t)stream;
+  Side side;
+  if (mlp) {
+    const cudaError_t es = side.create();
+    if (es != cudaSuccess) return cuda_fail(es, "setting up the side stream");
+  }
   // graphs are captured on a private non-blocking stream (the legacy default
   // stream cannot be captured), ordered after and before the caller's stream
   cudaStream_t s = caller;
@@ -183,15 +326,19 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   };
   auto run_slope0 = [&]() -> cudaError_t {
     cudaError_t e0 = with_pot([&](auto P) -> cudaError_t {
+      if (mlp) {
+        k_state0<<<grid, 256, 0, s>>>(P, y, F, Yq, A, n);
+        return launch_terms(P, Yq, F, A, n, mlp, s, side);
+      }
       k_slope0<<<grid, 256, 0, s>>>(P, y, F, Yq, n);
       return cudaSuccess;
     });
-    if (e0 != cudaSuccess) return e0;
-    if (mlp && gal_mlp_eval(mlp, Yq, n, F + 3 * n, 1, -1.0, nullptr, s) != GAL_OK) return cudaErrorLaunchFailure;
-    return cudaGetLastError();
+    return e0 != cudaSuccess ? e0 : cudaGetLastError();
   };
   auto run_step = [&](double hs) -> cudaError_t {
-    return with_pot([&](auto P) -> cudaError_t { return launch_step(P, y, F, Yq, hs, n, mlp, s, grid); });
+    return with_pot([&](auto P) -> cudaError_t {
+      return mlp ? launch_step_mlp(P, y, F, Yq, A, hs, n, mlp, s, side, grid) : launch_step(P, y, F, Yq, hs, n, s, grid);
+    });
   };
   if ((e = run_slope0()) != cudaSuccess) return finish(cuda_fail(e, "surrogate first slope"));
   cudaGraphExec_t exec = nullptr;
