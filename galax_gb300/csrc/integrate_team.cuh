@@ -22,8 +22,9 @@
 //   warp 2: the radius and the halo's factor;
 //   warp 3: the Miyamoto-Nagai disk (mw_disk);
 // warps 0-2 own state components (w, w + 3), form their stage states and
-// combine the pieces into their gradient component. Step control is computed
-// redundantly by all four warps from the same shared-memory values. Every
+// combine the pieces into their gradient component. Dopri5's step control is
+// computed redundantly by all four warps from the same shared-memory values;
+// Dopri8's by warp 2, while the others evaluate the slope at the step's end. Every
 // operation matches the one-thread-per-orbit kernel (k_integrate_mw with
 // MWPot::grad, integrate_loop), so results are bitwise identical.
 //
@@ -39,6 +40,8 @@
 // evaluation of its own.
 #pragma once
 
+#include <type_traits>
+
 #include "integrate.cuh"
 
 namespace gal {
@@ -48,8 +51,22 @@ struct TeamShared {
   double pos[3][32];
   // controller exchange
   double y1[6][kTeamLanes], err[6][kTeamLanes];
+  double next_t1[kTeamLanes], prev_inv[kTeamLanes], prev_prev_inv[kTeamLanes];
+  int flags[kTeamLanes];
   long long slot[kTeamLanes];
 };
+
+// A callable for a model's side job.
+template <class Fn>
+struct SideJob {
+  static constexpr bool any = true;
+  Fn fn;
+  __device__ __forceinline__ void operator()() const { fn(); }
+};
+template <class Fn>
+__device__ __forceinline__ SideJob<Fn> side_job(Fn fn) {
+  return SideJob<Fn>{fn};
+}
 
 // Y_j = y_j + hs sum_{l<I} A[I][l] F_l,j for one component (stage_state's
 // arithmetic): row IA on lanes 0-15, row IB on lanes 16-31. Zero coefficients
@@ -119,7 +136,12 @@ __device__ __forceinline__ double dense_comp(double y0j, double hs, const double
 
 // Models: grad() is one round of field evaluations, a point per lane, at time t.
 // The owners (warps 0-2) hold their position component q; warp w < 3 gets its
-// gradient component.
+// gradient component. With a side job, warp 2 does that between the two barriers
+// and the others take over its share where that is small.
+struct NoSide {
+  static constexpr bool any = false;
+  __device__ __forceinline__ void operator()() const {}
+};
 //
 // The Milky Way.
 struct TeamMW {
@@ -131,15 +153,26 @@ struct TeamMW {
   const MWParams& p;
   Shared& m;
 
-  __device__ __forceinline__ double grad(TeamShared& sh, int warp, int lane, double q, double) const {
+  template <class Side = NoSide>
+  __device__ __forceinline__ double grad(TeamShared& sh, int warp, int lane, double q, double,
+                                         Side&& side = Side{}) const {
+    constexpr bool busy = std::decay_t<Side>::any;  // warp 2 has a side job: warp 3 takes its factor
     if (warp < 3) sh.pos[warp][lane] = q;
     __syncthreads();  // positions written
     const double x = sh.pos[0][lane], y = sh.pos[1][lane], z = sh.pos[2][lane];
-    if (warp == 3) {
+    if (busy && warp == 2) {
+      side();
+    } else if (warp == 3) {
       const MWDisk d = mw_disk(p, x, y, z);
       m.u[lane] = d.u;
       m.us[lane] = d.us;
       m.izb[lane] = d.izb;
+      if constexpr (busy) {
+        double r;
+        const double ir = mw_ir(x, y, z, r);
+        m.A[lane] = p.Gm_h * (ir * ir);
+        m.ir[lane] = ir;
+      }
     } else {  // mw_f's products where their factors are
       double r;
       const double ir = mw_ir(x, y, z, r);
@@ -210,10 +243,13 @@ struct TeamTable {
     }
   }
 
-  __device__ __forceinline__ double grad(TeamShared& sh, int warp, int lane, double q, double t) const {
+  template <class Side = NoSide>
+  __device__ __forceinline__ double grad(TeamShared& sh, int warp, int lane, double q, double t,
+                                         Side&& side = Side{}) const {
     if (warp < 3) sh.pos[warp][lane] = q;
     __syncthreads();  // positions written
     const double x = sh.pos[0][lane], y = sh.pos[1][lane], z = sh.pos[2][lane];
+    if (std::decay_t<Side>::any && warp == 2) side();
     for (int i = 0; i < n; ++i) {
       if (m.warp[i] != warp) continue;
       const DevComp& c = m.c[i];
@@ -259,7 +295,7 @@ __device__ void team_loop(const IntegrateArgs& a, const Model& pot, const Blocks
   double yp = 0.0, yv = 0.0;  // owned position and velocity component (s.y holds all six for the controller)
   double np = 0.0, nv = 0.0;  // Dopri8: the same of the accepted end state while saves are pending
   double F0v = 0.0;           // owned velocity component of the slope at (tau, y); its position component is yv
-  bool need_f0 = false;       // Dopri8: the slope at a newly committed state is still to be evaluated
+  bool need_f0 = false;       // Dopri8: the slope at a state committed after its saves is still to be evaluated
   while (true) {
     // ---- orbits for free lanes (warp 0 dequeues)
     if (warp == 0 && !hi && need_orbit && queue_open) {
@@ -377,30 +413,67 @@ __device__ void team_loop(const IntegrateArgs& a, const Model& pot, const Blocks
     if (owner) {
       const bool want_err = a.adaptive && !sub;
       Fp[S - 1] = pair_row<TB, S - 1, S - 1>(hi, yv, hs, Fv);
+      double Fw[S];  // lanes 0-15 take the position's sums, lanes 16-31 the velocity's
+#pragma unroll
+      for (int l = 0; l < S; ++l) Fw[l] = hi ? Fv[l] : Fp[l];
+      double y1w;
       if constexpr (TB::FSAL) {
-        y1v = Fp[S - 1];
-        const double other = __shfl_xor_sync(0xffffffffu, y1p, kTeamLanes);
-        y1p = hi ? y1p : other;
+        y1w = hi ? Fp[S - 1] : y1p;
+        const double last = __shfl_xor_sync(0xffffffffu, y1p, kTeamLanes);
+        if (!hi) y1w = last;
       } else {
-        y1p = weighted_comp<TB, W_SOLUTION, true>(yp, hs, Fp);
-        y1v = weighted_comp<TB, W_SOLUTION, true>(yv, hs, Fv);
+        y1w = weighted_comp<TB, W_SOLUTION, true>(hi ? yv : yp, hs, Fw);
       }
-      sh.y1[jw][slot] = hi ? y1v : y1p;
-      if (want_err) {
-        double Fw[S];
+      const double other = __shfl_xor_sync(0xffffffffu, y1w, kTeamLanes);
+      y1p = hi ? other : y1w;
+      y1v = hi ? y1w : other;
+      sh.y1[jw][slot] = y1w;
+      if (want_err) sh.err[jw][slot] = weighted_comp<TB, W_ERROR, false>(0.0, hs, Fw);
+    }
+    // ---- step control (pid_adapt), and for Dopri8 the slope at the new state
+    // beside it: should the step be rejected, that round was in vain. With nothing
+    // to run beside, all warps do the control from the same values.
+    const bool control = a.adaptive && !sub && active;
+    double y1[6], next_t0 = 0.0, next_t1 = 0.0, F1v = 0.0;
+    bool keep = true;
+    auto read_y1 = [&]() {
 #pragma unroll
-        for (int l = 0; l < S; ++l) Fw[l] = hi ? Fv[l] : Fp[l];
-        sh.err[jw][slot] = weighted_comp<TB, W_ERROR, false>(0.0, hs, Fw);
+      for (int j = 0; j < 6; ++j) y1[j] = sh.y1[j][slot];
+    };
+    auto adapt = [&]() {
+      double err[6];
+#pragma unroll
+      for (int j = 0; j < 6; ++j) err[j] = sh.err[j][slot];
+      keep = pid_adapt<TB::ORDER>(a, s, y1, err, s.tnext - s.tau, next_t0, next_t1);
+    };
+    if constexpr (TB::FSAL) {
+      __syncthreads();
+      read_y1();
+      if (control) adapt();
+    } else {
+      F1v = -pot.grad(sh, warp, lane, active ? y1p : kIdle, Model::TIMED ? with_sign(s.dir, s.tnext) : 0.0,
+                      side_job([&]() {
+                        if (!control) return;
+                        read_y1();
+                        adapt();
+                        if (hi) return;
+                        sh.next_t1[slot] = next_t1;
+                        sh.prev_inv[slot] = s.prev_inv;
+                        sh.prev_prev_inv[slot] = s.prev_prev_inv;
+                        sh.flags[slot] = (keep ? 1 : 0) | (s.at_dtmin ? 2 : 0) | (s.status << 2);
+                      }));
+      read_y1();
+      if (control) {
+        const int flags = sh.flags[slot];
+        keep = (flags & 1) != 0;
+        s.at_dtmin = (flags >> 1) & 1;
+        s.status = flags >> 2;
+        s.prev_inv = sh.prev_inv[slot];
+        s.prev_prev_inv = sh.prev_prev_inv[slot];
+        next_t0 = keep ? s.tnext : s.tau;
+        next_t1 = sh.next_t1[slot];
       }
     }
-    __syncthreads();
-    double y1[6], err[6];
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      y1[j] = sh.y1[j][slot];
-      err[j] = a.adaptive ? sh.err[j][slot] : 0.0;
-    }
-    __syncthreads();  // the exchange arrays are reused next step
     if (!active) continue;
     bool done = false;
     int32_t st = ORBIT_OK;
@@ -419,13 +492,7 @@ __device__ void team_loop(const IntegrateArgs& a, const Model& pot, const Blocks
       s.tnext = s.tnext_new;
     } else {
       ++s.nsteps;
-      const double h = s.tnext - s.tau;
-      double next_t0, next_t1;
-      bool keep;
-      if (a.adaptive) {
-        keep = pid_adapt<TB::ORDER>(a, s, y1, err, h, next_t0, next_t1);
-      } else {
-        keep = true;
+      if (!a.adaptive) {
         next_t0 = s.tnext;
         next_t1 = s.tnext + a.dt0;
       }
@@ -442,7 +509,7 @@ __device__ void team_loop(const IntegrateArgs& a, const Model& pot, const Blocks
           ++s.naccepted;
           if (s.save_i < s.save_end && le_bits(save_tau(a, s, s.save_i), next_t0)) {
             if constexpr (TB::FSAL) {
-              const double ih = 1.0 / h;
+              const double ih = 1.0 / (s.tnext - s.tau);
               double Fw[S];
 #pragma unroll
               for (int l = 0; l < S; ++l) Fw[l] = hi ? Fv[l] : Fp[l];
@@ -473,8 +540,7 @@ __device__ void team_loop(const IntegrateArgs& a, const Model& pot, const Blocks
           for (int j = 0; j < 6; ++j) s.y[j] = y1[j];
           yp = y1p;
           yv = y1v;
-          if constexpr (TB::FSAL) F0v = Fv[S - 1];
-          need_f0 = !TB::FSAL;
+          F0v = TB::FSAL ? Fv[S - 1] : F1v;
         }
         s.tau = tprev_new;
         s.tnext = tnext_new;
