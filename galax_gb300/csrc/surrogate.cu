@@ -1,13 +1,13 @@
 // Orbit integration with the learned surrogate: analytic FP64 part + MLP part.
 //
 // Dopri5 with a constant step over a batch of orbits, stepped at batch level. Per
-// stage one kernel forms the stage state Y = y + h sum_l a_il F_l, its positions
-// and the near field there; the tensor-core MLP kernel and the FP64 kernel of the
-// analytic part then evaluate the two terms of F_i = (Y_v, -grad Phi(Y_q)) side by
-// side. The seventh stage is evaluated at y_{n+1} (FSAL), so it becomes the next
-// step's first slope in place. One step is captured once as a CUDA graph and
-// replayed. Without a network, one kernel per stage does it all. The analytic part
-// is any gal_potential (the Milky Way model runs its specialised gradient).
+// stage one FP64 kernel forms the stage state Y = y + h sum_l a_il F_l, writes
+// F_i = (Y_v, -grad Phi_analytic(Y_q)) and the stage positions, and the tensor-core
+// MLP kernel adds -grad Phi_MLP(Y_q) into F_i; without a near field the two terms
+// are evaluated side by side. The seventh stage is evaluated at y_{n+1} (FSAL), so
+// it becomes the next step's first slope in place. One step is captured once as a
+// CUDA graph and replayed. The analytic part is any gal_potential (the Milky Way
+// model runs its specialised gradient).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -84,30 +84,26 @@ __global__ void __launch_bounds__(256) k_slope0(Pot pot, const double* __restric
   }
 }
 
-// With a network, a stage is three kernels. k_state forms the stage state from the
-// slopes and sums the near field there; then the network's term (tensor cores) and
-// the analytic one (FP64) are evaluated side by side, the one into the slope's own
-// place, the other into A [3][n], onto the near field; the next k_state adds the
-// two, A first, and leaves the sum as the slope. The network kernel holds each SM's
-// shared memory, and with it all but a few KB of L1, and all but 11,776 of its
-// registers; the analytic kernel's one block of two warps per SM fits into these
-// and passes under the network's time. (The near field does not: its lists need the
-// L1 and many warps, 54 ms for the steps below.) 131,072 orbits, 20 steps, with a
-// near field of 512 spheres: 23.7 -> 20.9 ms; without: 18.8 -> 16.6 ms; 500 orbits: 8.6
-// -> 5.6 ms.
+// With a network and no near field, a stage is three kernels. k_state forms the
+// stage state from the slopes; then the network's term (tensor cores) and the
+// analytic one (FP64) are evaluated side by side, the one into the slope's own
+// place, the other into A [3][n]; the next k_state adds the two, A first, and leaves
+// the sum as the slope. The network kernel holds each SM's shared memory, and with
+// it all but a few KB of L1, and all but 11,776 of its registers; the analytic
+// kernel's one block of two warps per SM fits into these and passes under the
+// network's time. 131,072 orbits, 20 steps: 18.8 -> 16.6 ms. A near field does not
+// fit there (its lists need the L1 and many warps: 54 ms instead of 23.5), and summed
+// apart by groups of lanes (20.5 ms) its FP32 terms come in another order, which the
+// network's roundings make visible; it stays in the fused stage kernel.
 //
 // Stage I of a step from (y, F): as k_stage, without the gradient; P is the slot of
 // the previous stage, whose two terms are still apart.
-template <int I, class Pot>
-__global__ void __launch_bounds__(256) k_state(Pot pot, double* __restrict__ y, double* __restrict__ F,
+template <int I>
+__global__ void __launch_bounds__(256) k_state(double* __restrict__ y, double* __restrict__ F,
                                                double* __restrict__ Yq, double* __restrict__ A, double hs, int64_t n) {
   constexpr int P = I - 1;
   constexpr int slot = (I == Dopri5::S - 1) ? 0 : I;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t first = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); first < n; first += stride) {
-    const int64_t own = first + (threadIdx.x & 31);
-    const bool valid = own < n;
-    const int64_t i = valid ? own : n - 1;  // the last warp's spare lanes follow its last orbit and write nothing
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double Y[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
@@ -126,19 +122,12 @@ __global__ void __launch_bounds__(256) k_state(Pot pot, double* __restrict__ y, 
       });
       Y[j] = fma(hs, acc, y[(int64_t)j * n + i]);
     }
-    float near[3];
-    const bool has_near = near_grad(pot, Y[0], Y[1], Y[2], near);
-    if (!valid) continue;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const int64_t a = ((int64_t)P * 6 + 3 + j) * n + i;
       F[a] = A[j * n + i] + F[a];  // the slope itself, for the later stages
       F[((int64_t)slot * 6 + j) * n + i] = Y[3 + j];
       Yq[(int64_t)j * n + i] = Y[j];
-    }
-    if (has_near) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) A[(int64_t)j * n + i] = (double)near[j];
     }
     if constexpr (I == Dopri5::S - 1) {
 #pragma unroll
@@ -147,23 +136,14 @@ __global__ void __launch_bounds__(256) k_state(Pot pot, double* __restrict__ y, 
   }
 }
 
-// The first step's first slope: its position, velocity part and near field.
-template <class Pot>
-__global__ void __launch_bounds__(256) k_state0(Pot pot, const double* __restrict__ y, double* __restrict__ F,
-                                                double* __restrict__ Yq, double* __restrict__ A, int64_t n) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t first = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); first < n; first += stride) {
-    const int64_t own = first + (threadIdx.x & 31);
-    const int64_t i = own < n ? own : n - 1;
-    const double x[3] = {y[i], y[n + i], y[2 * n + i]};
-    float near[3];
-    const bool has_near = near_grad(pot, x[0], x[1], x[2], near);
-    if (own >= n) continue;
+// The first step's first slope: its position and velocity part.
+__global__ void __launch_bounds__(256) k_state0(const double* __restrict__ y, double* __restrict__ F,
+                                                double* __restrict__ Yq, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       F[(int64_t)j * n + i] = y[(int64_t)(3 + j) * n + i];
-      Yq[(int64_t)j * n + i] = x[j];
-      if (has_near) A[(int64_t)j * n + i] = (double)near[j];
+      Yq[(int64_t)j * n + i] = y[(int64_t)j * n + i];
     }
   }
 }
@@ -172,18 +152,15 @@ __global__ void __launch_bounds__(256) k_state0(Pot pot, const double* __restric
 // each of two sub-partitions, two on the others): at most 168 registers.
 constexpr int kAnalyticBlock = 64;
 
-// A: -(analytic gradient + the near field that k_state left there).
 template <class Pot>
 __global__ void __launch_bounds__(kAnalyticBlock, 6) k_analytic(Pot pot, const double* __restrict__ Yq,
                                                                 double* __restrict__ A, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double g[3];
-    const bool has_near = far_grad(pot, Yq[i], Yq[n + i], Yq[2 * n + i], g);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      if (has_near) g[j] += A[j * n + i];
-      A[j * n + i] = -g[j];
-    }
+    double gx, gy, gz;
+    pot.grad(Yq[i], Yq[n + i], Yq[2 * n + i], gx, gy, gz);
+    A[i] = -gx;
+    A[n + i] = -gy;
+    A[2 * n + i] = -gz;
   }
 }
 
@@ -230,19 +207,25 @@ static cudaError_t launch_step_mlp(const Pot& pot, double* y, double* F, double*
   static_for<1, Dopri5::S>([&](auto i) {
     constexpr int I = decltype(i)::value;
     if (e != cudaSuccess) return;
-    k_state<I><<<grid, 256, 0, s>>>(pot, y, F, Yq, A, hs, n);
+    k_state<I><<<grid, 256, 0, s>>>(y, F, Yq, A, hs, n);
     e = launch_terms(pot, Yq, F + (int64_t)(I == Dopri5::S - 1 ? 0 : I) * 6 * n, A, n, mlp, s, side);
   });
   return e;
 }
 
+// The fused stage kernel, and the network's term added by its own.
 template <class Pot>
-static cudaError_t launch_step(const Pot& pot, double* y, double* F, double* Yq, double hs, int64_t n, cudaStream_t s,
-                               unsigned grid) {
+static cudaError_t launch_step(const Pot& pot, double* y, double* F, double* Yq, double hs, int64_t n,
+                               const gal_mlp* mlp, cudaStream_t s, unsigned grid) {
+  cudaError_t e = cudaSuccess;
   static_for<1, Dopri5::S>([&](auto i) {
-    k_stage<decltype(i)::value><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
+    constexpr int I = decltype(i)::value;
+    if (e != cudaSuccess) return;
+    k_stage<I><<<grid, 256, 0, s>>>(pot, y, F, Yq, hs, n);
+    double* slot = F + (int64_t)(I == Dopri5::S - 1 ? 0 : I) * 6 * n;
+    if (mlp && gal_mlp_eval(mlp, Yq, n, slot + 3 * n, 1, -1.0, nullptr, s) != GAL_OK) e = cudaErrorLaunchFailure;
   });
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -274,7 +257,9 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   double* A = reinterpret_cast<double*>(reinterpret_cast<char*>(Yq) + align256(sizeof(double) * 3 * (size_t)n));
   cudaStream_t caller = (cudaStream_t)stream;
   Side side;
-  if (mlp) {
+  const SplitDev* spd = gal_split_device(near);
+  const bool apart = mlp && !spd;  // network and analytic term side by side
+  if (apart) {
     const cudaError_t es = side.create();
     if (es != cudaSuccess) return cuda_fail(es, "setting up the side stream");
   }
@@ -315,7 +300,6 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   const unsigned grid = (unsigned)(grid64 > cap ? cap : grid64);
   cudaError_t e;
   // the analytic part, with the exact short-range Plummer sum when a split is given
-  const SplitDev* spd = gal_split_device(near);
   auto with_pot = [&](auto&& fn) -> cudaError_t {
     if (pot->is_mw) {
       const MWPot base{pot->mw};
@@ -326,18 +310,20 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   };
   auto run_slope0 = [&]() -> cudaError_t {
     cudaError_t e0 = with_pot([&](auto P) -> cudaError_t {
-      if (mlp) {
-        k_state0<<<grid, 256, 0, s>>>(P, y, F, Yq, A, n);
+      if (apart) {
+        k_state0<<<grid, 256, 0, s>>>(y, F, Yq, n);
         return launch_terms(P, Yq, F, A, n, mlp, s, side);
       }
       k_slope0<<<grid, 256, 0, s>>>(P, y, F, Yq, n);
+      if (mlp && gal_mlp_eval(mlp, Yq, n, F + 3 * n, 1, -1.0, nullptr, s) != GAL_OK) return cudaErrorLaunchFailure;
       return cudaSuccess;
     });
     return e0 != cudaSuccess ? e0 : cudaGetLastError();
   };
   auto run_step = [&](double hs) -> cudaError_t {
     return with_pot([&](auto P) -> cudaError_t {
-      return mlp ? launch_step_mlp(P, y, F, Yq, A, hs, n, mlp, s, side, grid) : launch_step(P, y, F, Yq, hs, n, s, grid);
+      return apart ? launch_step_mlp(P, y, F, Yq, A, hs, n, mlp, s, side, grid)
+                   : launch_step(P, y, F, Yq, hs, n, mlp, s, grid);
     });
   };
   if ((e = run_slope0()) != cudaSuccess) return finish(cuda_fail(e, "surrogate first slope"));

@@ -1,8 +1,7 @@
-"""The surrogate's stages with a network (near field by groups of lanes, network
-and analytic term side by side) against the stage kernel without one: a network
-of zeros adds nothing, so the two differ by the order of the near field's FP32
-sums. Batches with partial warps, points beyond the near field's cells, captured
-and direct launches."""
+"""The surrogate's stages with a network (beside the analytic term where there is
+no near field) against the stage kernel without one: a network of zeros adds
+nothing. Batches with partial warps, points beyond the near field's cells,
+captured and direct launches."""
 
 import numpy as np
 import pytest
@@ -35,8 +34,4 @@ def test_zero_network_adds_nothing(n, with_near, host):
     got = S.integrate(pot, mlp, y0, 0.0, 10.0, 1.0, near=near)
     direct = S.integrate(pot, mlp, y0, 0.0, 10.0, 1.0, near=near, use_graph=False)
     assert torch.equal(got, direct)
-    if with_near:
-        # 60 FP32 terms of at most 2e-3 kpc/Myr^2, 2^-24 each, over 10 Myr: below 1e-6 in velocity and position
-        assert float((got - plain).abs().max()) < 1e-6
-    else:
-        assert torch.equal(got, plain)
+    assert torch.equal(got, plain)
