@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(128) k_adjoint(AdjointArgs a, Pot pot, const D
 //   dL/dtheta += sum_i gbar_i . (dg/dtheta)(X_i).
 // The scratch holds the stages of `seg` steps; longer spans are cut into such
 // segments, and all but the last are integrated a second time from their first
-// state. FP64 instructions per Dopri8 step: 2,960 (4,240 with segments), where
-// k_adjoint takes 8,260 (three forward evaluations and four separate components).
+// state. FP64 instructions per Dopri8 step: about 2,700 (3,900 with segments), where
+// k_adjoint takes 7,900 (three forward evaluations and four separate components).
 // 16,384 orbits, 500 steps: 143.5 -> 48.0 ms.
 constexpr int kStageDoubles = 10;
 

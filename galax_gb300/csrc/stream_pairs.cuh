@@ -140,7 +140,7 @@ __device__ __forceinline__ void stream_pair_step(const Team& team, int warp, int
   }
 }
 
-// The progenitor in a Milky Way host: one orbit, the same in every slot. 15 us
+// The progenitor in a Milky Way host: one orbit, the same in every slot. 14 us
 // instead of 26 per Dopri8 step.
 template <class TB>
 __global__ void __launch_bounds__(128) k_stream_progenitor_mw(StreamDev a, MWParams p) {
