@@ -43,11 +43,9 @@ def set_launch(method: int, adaptive: bool, block: int, per_sm: int, variant: in
 
 # SMs given to four-warp teams for the longest orbits (second pass of a
 # two-pass adaptive Milky Way batch, gal_set_team), per method. On the
-# 262,144-orbit headline batch the step time has a narrow minimum, so the
-# candidates are spaced closely around it (ms, Dopri5: 24 -> 1,253,
-# 28 -> 1,171, 30 -> 1,172, 32 -> 1,183, 36 -> 1,211, 40 -> 1,241; Dopri8:
-# 2 -> 1,590, 4 -> 1,525, 6 -> 1,500, 8 -> 1,454, 12 -> 1,474, 16 -> 1,499,
-# 24 -> 1,549, 32 -> 1,609, none -> 1,852).
+# 262,144-orbit headline batch (ms, Dopri5: 24 -> 1,175, 28 -> 1,100, 32 -> 1,102,
+# 40 -> 1,113; Dopri8: 6 -> 1,430, 8 -> 1,431, 10 -> 1,422, 12 -> 1,431,
+# 16 -> 1,429, none -> 1,887).
 DEFAULT_TEAMS = {5: (24, 28, 32, 40), 8: (6, 8, 10, 12, 16)}
 
 

@@ -278,7 +278,7 @@ __device__ __forceinline__ int sym_index(int a, int b) {
 constexpr int kSweepParticles = 5;  // particles per warp
 
 // Reverse sweep with the stored Hessians, five particles per warp; the next
-// step's Hessian rows are loaded a step ahead. 4 us instead of 41 per Dopri8 step.
+// step's Hessian rows are loaded a step ahead. 5 us instead of 41 per Dopri8 step.
 template <class TB>
 __global__ void __launch_bounds__(32) k_stream_particles_sweep(StreamDev a) {
   constexpr int S = TB::S, R = PairSweep<TB>::R;
