@@ -101,52 +101,18 @@ static MWParams mw_params(const gal_component* c, double G) {
   return p;
 }
 
-// The table's Plummer spheres in fixed point (fixed_plummer.cuh), where their
-// scales fit; p->fixed.n = 0 otherwise. Allocates on the first call for a handle
-// (the number of components never changes).
+// The table's Plummer spheres in fixed point (fixed_plummer.cuh), if they are
+// many; p->fixed.n = 0 otherwise. Allocates on the first call for a handle (the
+// number and kinds of components never change).
 static cudaError_t build_fixed(gal_potential* p) {
   p->fixed = FixedTable{};
   std::vector<int32_t> at, other;
-  double reach = 0.0;
-  for (int i = 0; i < p->n; ++i) {
-    const gal_component& c = p->comps[i];
-    if (c.kind != GAL_PLUMMER) {
-      other.push_back(i);
-      continue;
-    }
-    at.push_back(i);
-    for (double v : c.origin) reach = std::fmax(reach, std::fabs(v));
-    reach = std::fmax(reach, c.l1);
-  }
-  if ((int)at.size() < kWarpMinComponents || !(reach > 0.0)) return cudaSuccess;
-  int top = 0;
-  std::frexp(reach, &top);       // reach <= 2^top
-  const int xtop = top + 2;      // positions up to 2^xtop: offsets below 2^(xtop + 1)
-  const int s = 60 - 1 - xtop;   // ... and below 2^60 in units of 2^-s
-  if (std::abs(s) > 900) return cudaSuccess;
+  for (int i = 0; i < p->n; ++i) (p->comps[i].kind == GAL_PLUMMER ? at : other).push_back(i);
+  if ((int)at.size() < kWarpMinComponents) return cudaSuccess;
   std::vector<FixedPlummer> h(at.size());
   for (size_t i = 0; i < at.size(); ++i) {
     const gal_component& c = p->comps[at[i]];
-    FixedPlummer& f = h[i];
-    f = FixedPlummer{};
-    for (int j = 0; j < 3; ++j) f.c[j] = std::llrint(std::ldexp(c.origin[j], s));
-    const double Gm = p->G * c.m;
-    int e = 0;
-    f.gm = (uint64_t)std::ldexp(std::frexp(std::fabs(Gm), &e), 64);
-    f.sign = Gm < 0.0 ? 0x80000000u : 0u;
-    f.e0 = (e - 64) - 178 + 2 * s;
-    if (f.gm != 0 && (f.e0 < -1000 || f.e0 > 800)) return cudaSuccess;  // the result's exponent stays normal
-    if (c.l1 > 0.0) {
-      const double b = std::ldexp(c.l1, s);
-      f.bhi = (uint32_t)((uint64_t)b >> 32);
-      int eb = 0;
-      const double m = std::frexp(b, &eb);  // b = m 2^eb; 2^kb b in [2^60, 2^61)
-      f.kb = 61 - eb;
-      if (f.kb > 1000) return cudaSuccess;
-      const uint64_t n = (uint64_t)std::ldexp(m, 53);  // exact; b2 = (n 2^8)^2 / 2^60 = n^2 / 2^44
-      const uint64_t hi = n >> 32, lo = n & 0xffffffffu;
-      f.b2 = (hi * hi << 20) + ((hi * lo) >> 11) + ((lo * lo) >> 44);
-    }
+    h[i] = fixed_record(c.origin, c.l1, p->G * c.m);
   }
   at.insert(at.end(), other.begin(), other.end());
   const size_t records = sizeof(FixedPlummer) * h.size();
@@ -164,9 +130,6 @@ static cudaError_t build_fixed(gal_potential* p) {
   p->fixed.at = reinterpret_cast<const int32_t*>(base + records);
   p->fixed.n = (int)h.size();
   p->fixed.nother = (int)other.size();
-  p->fixed.s = s;
-  p->fixed.scale = std::ldexp(1.0, s);
-  p->fixed.xmax = std::ldexp(1.0, xtop);
   gal_component four[4];
   p->fixed_mw = other.size() == 4;
   for (size_t i = 0; i < other.size() && i < 4; ++i) four[i] = p->comps[other[i]];

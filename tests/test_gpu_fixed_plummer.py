@@ -70,3 +70,39 @@ def test_fixed_point_spheres_match_fp64(method, k, others, n):
         want = np.stack(ref).transpose(2, 1, 0)
         s = np.linalg.norm(want.reshape(2, 3, *want.shape[1:]), axis=1, keepdims=True)
         assert np.max(np.abs(a[:, :, 4:] - want).reshape(2, 3, *want.shape[1:]) / s) < 1e-9
+
+
+@pytest.mark.parametrize("method", [5, 8])
+@pytest.mark.parametrize("reach,b", [(50.0, 0.1), (50.0, 1e-3), (800.0, 0.01), (1e5, 0.01), (1e5, 1e-4)])
+def test_near_a_sphere_of_a_wide_table(method, reach, b):
+    """Orbits at rest within a few scales of one sphere, the others far away and as
+    extended: the velocity after one short step is the gradient's error alone. FP64's
+    own is some 10 roundings of 2^-53 per gradient, the fixed-point one's 5; the
+    weights' sizes add up to 3.1 (Dopri8) with a rounding of each term: below 1e-14
+    together."""
+    import galax_gb300 as gx
+    from galax_gb300 import _lib
+    from galax_gb300.dynamics import integrate
+
+    L = _lib.load()
+    rng = np.random.default_rng(9)
+    c0 = np.array([8.0, 1.0, -2.0])
+    far = rng.normal(size=(40, 3))
+    far *= reach / np.linalg.norm(far, axis=1, keepdims=True)
+    pot = gx.CompositePotential([gx.PlummerPotential(m_tot=1e9, r_s=b, origin=tuple(c0))] + [
+        gx.PlummerPotential(m_tot=1e6, r_s=0.1 * reach, origin=tuple(c)) for c in far])
+    x = rng.normal(size=(200, 3))
+    x *= b * rng.uniform(0.3, 3.0, (200, 1)) / np.linalg.norm(x, axis=1, keepdims=True)
+    y0 = np.concatenate([c0 + x, np.zeros((200, 3))], axis=1)
+    dt = 1e-3 * np.sqrt(b**3 / (4.5e-12 * 1e9))  # a thousandth of the sphere's own time
+    cfg = gx.Integrator(solver=gx.Dopri8() if method == 8 else gx.Dopri5(),
+                        stepsize_controller=gx.ConstantStepSize(), dt0=dt).config()
+    try:
+        fixed = integrate(pot, y0, 0.0, dt, np.array([dt]), cfg)[0].cpu().numpy()
+        _lib.check(L.gal_set_table_lanes(1), "gal_set_table_lanes")
+        fp64 = integrate(pot, y0, 0.0, dt, np.array([dt]), cfg)[0].cpu().numpy()
+    finally:
+        _lib.check(L.gal_set_table_lanes(0), "gal_set_table_lanes")
+    v, w = fixed[3:, 0], fp64[3:, 0]
+    assert np.all(np.abs(w).max(axis=0) > 0)
+    assert np.max(np.linalg.norm(v - w, axis=0) / np.linalg.norm(w, axis=0)) < 1e-14
