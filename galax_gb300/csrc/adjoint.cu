@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(32) k_adjoint_mw(StoredArgs a, MWParams p, con
         const double hl = h * lx[j], l = lv[j];
         static_for<0, S>([&](auto i) {
           constexpr int I = decltype(i)::value;
-          constexpr double cx = kNystrom<TB>.b[I], cv = TB::B[I];
+          constexpr double cx = kNystrom<TB>.b[I], cv = kNystrom<TB>.v[I];
           if constexpr (cx != 0.0 && cv != 0.0) G[I][j] = fma(cx, hl, cv * l);
           else if constexpr (cx != 0.0) G[I][j] = cx * hl;
           else if constexpr (cv != 0.0) G[I][j] = cv * l;

@@ -6,6 +6,7 @@ import ctypes as C
 import shutil
 import subprocess
 from decimal import Decimal, getcontext
+from fractions import Fraction
 from pathlib import Path
 
 import numpy as np
@@ -85,3 +86,45 @@ def test_fixed_point_leaves_the_ends_of_the_range_to_fp64(tmp_path):
     assert not fits((0, 0, 0), 1.0, 1e61, (1, 0, 0)) and not fits((0, 0, 0), 1.0, 1e-61, (1, 0, 0))
     for bad in (nan, inf, -inf):
         assert not fits((0, 0, 0), 1.0, 1.0, (0, bad, 0))
+
+
+NYSTROM = r"""
+#include <cmath>
+using std::fma;
+#include "nystrom.cuh"
+using namespace gal;
+template <class TB>
+static void table(double* a, double* b, double* v) {
+  for (int i = 0; i < TB::S; ++i) {
+    for (int l = 0; l < TB::S; ++l) *a++ = kNystrom<TB>.a[i][l];
+    *b++ = kNystrom<TB>.b[i];
+    *v++ = kNystrom<TB>.v[i];
+  }
+}
+extern "C" void nystrom(int method, double* a, double* b, double* v) {
+  if (method == 8) table<Dopri8>(a, b, v);
+  else table<Dopri5>(a, b, v);
+}
+"""
+
+
+@pytest.mark.parametrize("method", [5, 8])
+def test_nystrom_coefficients_are_rounded_once(tmp_path, method):
+    """abar = A A and bbar = b A to one rounding (2^-53 relative) or exactly zero,
+    and velocity weights next to b whose sum is 1 exactly."""
+    from oracle import oracle as O
+
+    S = 13 if method == 8 else 7
+    a, b, v = np.empty((S, S)), np.empty(S), np.empty(S)
+    _compile(tmp_path, NYSTROM).nystrom(method, *(w.ctypes.data_as(C.c_void_p) for w in (a, b, v)))
+    _, A, B, _ = O.tableau(method)[-4:]
+    exact = np.vectorize(Fraction)
+    A, B = exact(A[:S, :S]), exact(B[:S])
+    want_a, want_b = A @ A, B @ A
+    for got, want in zip(np.append(a, b), np.append(want_a, want_b)):
+        if got == 0.0:
+            assert abs(want) < 1e-15
+        else:
+            assert abs(Fraction(float(got)) - want) <= abs(want) * Fraction(1, 2**53)
+    assert sum(exact(v)) == 1
+    assert np.all(np.abs(v - B.astype(float)) <= np.spacing(np.abs(v)))
