@@ -114,27 +114,35 @@ static cudaError_t build_fixed(gal_potential* p) {
     const gal_component& c = p->comps[at[i]];
     h[i] = fixed_record(c.origin, c.l1, p->G * c.m);
   }
+  FixedOthers o{};
+  if (other.size() == 4) {
+    gal_component four[4];
+    for (int i = 0; i < 4; ++i) four[i] = p->comps[other[i]];
+    o.is_mw = milky_way_shape(four, 4) ? 1 : 0;
+    if (o.is_mw) o.mw = mw_params(four, p->G);
+  }
   at.insert(at.end(), other.begin(), other.end());
-  const size_t records = sizeof(FixedPlummer) * h.size();
+  // records, the others' values, indices: one copy, so that a launch finds them all as they were or as they are
+  const size_t records = sizeof(FixedPlummer) * h.size(), values = 128;
+  static_assert(sizeof(FixedOthers) <= 128, "FixedOthers");
+  std::vector<char> image(records + values + sizeof(int32_t) * at.size());
+  std::memcpy(image.data(), h.data(), records);
+  std::memcpy(image.data() + records, &o, sizeof(o));
+  std::memcpy(image.data() + records + values, at.data(), sizeof(int32_t) * at.size());
   cudaError_t e = cudaSuccess;
-  if (!p->d_fixed) e = cudaMalloc(&p->d_fixed, sizeof(FixedPlummer) * (size_t)p->n + sizeof(int32_t) * (size_t)p->n);
+  if (!p->d_fixed) e = cudaMalloc(&p->d_fixed, image.size());
   if (e != cudaSuccess) {
     p->d_fixed = nullptr;
     return e;
   }
-  char* base = static_cast<char*>(p->d_fixed);
-  e = cudaMemcpy(base, h.data(), records, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(base + records, at.data(), sizeof(int32_t) * at.size(), cudaMemcpyHostToDevice);
+  e = cudaMemcpy(p->d_fixed, image.data(), image.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return e;
+  char* base = static_cast<char*>(p->d_fixed);
   p->fixed.f = reinterpret_cast<const FixedPlummer*>(base);
-  p->fixed.at = reinterpret_cast<const int32_t*>(base + records);
+  p->fixed.others = reinterpret_cast<const FixedOthers*>(base + records);
+  p->fixed.at = reinterpret_cast<const int32_t*>(base + records + values);
   p->fixed.n = (int)h.size();
   p->fixed.nother = (int)other.size();
-  gal_component four[4];
-  p->fixed_mw = other.size() == 4;
-  for (size_t i = 0; i < other.size() && i < 4; ++i) four[i] = p->comps[other[i]];
-  p->fixed_mw = p->fixed_mw && milky_way_shape(four, 4);
-  p->fixed_mwp = p->fixed_mw ? mw_params(four, p->G) : MWParams{};
   return cudaSuccess;
 }
 
@@ -711,8 +719,6 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   a.n = n;
   a.lin = p->d_lin;
   a.fixed = p->fixed;
-  a.fixed_mw = p->fixed_mw ? 1 : 0;
-  a.fixed_mwp = p->fixed_mwp;
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = static_cast<char*>(workspace);
   a.queue = reinterpret_cast<unsigned long long*>(ws);

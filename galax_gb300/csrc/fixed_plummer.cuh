@@ -167,9 +167,18 @@ __host__ __device__ __forceinline__ bool fixed_plummer(const FixedPlummer& p, co
 
 namespace gal {
 
+// What the other components are, with the spheres' records in device memory: a
+// graph captured with the table sees the values of the last gal_potential_update,
+// as it does through the component table. Counts and kinds never change.
+struct FixedOthers {
+  MWParams mw;
+  int32_t is_mw;  // a Milky Way's four
+};
+
 struct FixedTable {
   const FixedPlummer* f;  // spheres, in the order of the table's Plummer entries
-  const int32_t* at;      // their table indices, then those of the other components
+  const FixedOthers* others;
+  const int32_t* at;      // the spheres' table indices, then those of the other components
   int n, nother;
 };
 
@@ -180,11 +189,10 @@ struct FixedTable {
 struct FixedTablePot {
   const FixedPlummer* f;   // shared memory
   const DevComp* others;   // shared memory
+  const FixedOthers* o;    // shared memory
   const DevComp* comps;    // the whole table, for spheres out of range
   FixedTable t;
   int lanes;
-  bool mw;
-  MWPot milky_way;
 
   __device__ __forceinline__ void grad(double x, double y, double z, double& gx, double& gy, double& gz) const {
     const int sub = threadIdx.x & (lanes - 1);
@@ -208,6 +216,7 @@ struct FixedTablePot {
         if (!fixed_plummer(f[i], X, &w, d)) comp_grad(comps[t.at[i]], x, y, z, ax, ay, az);
       }
     }
+    const bool mw = o->is_mw != 0;
     if (!mw)
       for (int i = sub; i < t.nother; i += lanes) comp_grad(others[i], x, y, z, ax, ay, az);
     const unsigned mask = lanes >= 32 ? 0xffffffffu : ((1u << lanes) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(lanes - 1));
@@ -218,7 +227,7 @@ struct FixedTablePot {
     }
     if (mw) {
       double hx, hy, hz;
-      milky_way.grad(x, y, z, hx, hy, hz);
+      MWPot{o->mw}.grad(x, y, z, hx, hy, hz);
       ax += hx;
       ay += hy;
       az += hz;

@@ -18,10 +18,8 @@ struct gal_potential {
   bool is_mw;             // evaluated by the specialised Milky Way model
   gal::MWParams mw;
   gal::DevLinear* d_lin = nullptr;  // linear time dependence per component (NULL: static)
-  void* d_fixed = nullptr;          // FixedPlummer records and component indices (NULL: few spheres)
+  void* d_fixed = nullptr;          // records and indices of `fixed` (NULL: few spheres)
   gal::FixedTable fixed{};          // n = 0: not used
-  bool fixed_mw = false;            // the other components are a Milky Way's four
-  gal::MWParams fixed_mwp{};
 };
 
 namespace gal {

@@ -114,8 +114,6 @@ struct IntegrateArgs {
   unsigned long long* queue;  // work-queue counter (scratch)
   const DevLinear* lin;       // time-dependent component parameters (table kernel), or NULL
   FixedTable fixed;           // the table's Plummer spheres in fixed point (n = 0: not used)
-  int32_t fixed_mw;           // its other components are the Milky Way's four
-  MWParams fixed_mwp;
   // two-phase schedule: phase 0 parks every orbit once it has covered split_frac
   // of its span; phase 1 resumes the parked orbits from `resume` in `order`
   int32_t phase;

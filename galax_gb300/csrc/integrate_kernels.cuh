@@ -177,13 +177,14 @@ cudaError_t launch_integrate_warp(const IntegrateArgs& a, const DevComp* comps, 
 template <class TB>
 __global__ void __launch_bounds__(128, 4) k_integrate_fixed(IntegrateArgs a, const DevComp* comps, int lanes) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ FixedOthers others;
   FixedPlummer* s_f = reinterpret_cast<FixedPlummer*>(smem_raw);
   DevComp* s_o = reinterpret_cast<DevComp*>(s_f + a.fixed.n);
   for (int i = threadIdx.x; i < a.fixed.n; i += blockDim.x) s_f[i] = a.fixed.f[i];
   for (int i = threadIdx.x; i < a.fixed.nother; i += blockDim.x) s_o[i] = comps[a.fixed.at[a.fixed.n + i]];
+  if (threadIdx.x == 0) others = *a.fixed.others;
   __syncthreads();
-  integrate_loop<TB, FixedTablePot, 0>(
-      a, FixedTablePot{s_f, s_o, comps, a.fixed, lanes, a.fixed_mw != 0, MWPot{a.fixed_mwp}});
+  integrate_loop<TB, FixedTablePot, 0>(a, FixedTablePot{s_f, s_o, &others, comps, a.fixed, lanes});
 }
 
 template <class TB>
