@@ -223,14 +223,42 @@ __global__ void k_eval_phi(const DevComp* comps, const DevLinear* lin, double t,
   }
 }
 
+__device__ __forceinline__ void eval_hessian(const DevComp* s, int ncomp, const Points& x, int64_t n,
+                                             double* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int c = 0; c < ncomp; ++c) comp_hessian(s[c], x(i, 0), x(i, 1), x(i, 2), H);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) out[k * n + i] = H[k];
+  }
+}
+
+__global__ void k_eval_hessian(const DevComp* comps, const DevLinear* lin, double t, int ncomp, Points x, int64_t n,
+                               double* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  DevComp* s = reinterpret_cast<DevComp*>(smem_raw);
+  stage_at_time(comps, lin, ncomp, t, s);
+  __syncthreads();
+  eval_hessian(s, ncomp, x, n, out);
+}
+
 // The Milky Way's Hessian, FP64-bound: one radius, one logarithm and one
 // reciprocal for the three spheres, reciprocal square roots instead of roots and
 // quotients, and the six distinct entries, where the component table's general
 // code takes a root per component, about a dozen quotients and nine entries.
 // Positions are read where they are instead of from a transposed copy. 4,194,304
-// points: 2.23 -> 0.80 ms (relative error 1.8e-15 against 64-bit torch, 1.5e-15
-// before).
-__global__ void __launch_bounds__(128) k_eval_hessian_mw(MWParams p, Points x, int64_t n, double* __restrict__ out) {
+// points: 2.23 -> 0.80 ms. Against extended precision, of |H| at 200,000 points:
+// rms error 3.4e-16 (3.5e-16 by the general code), largest 3.7e-15 (5.7e-15).
+// The parameters come from the component table in device memory, so that a
+// captured call sees gal_potential_update; one that moved a component off the centre
+// leaves the general code.
+__global__ void __launch_bounds__(128) k_eval_hessian_mw(const DevComp* comps, Points x, int64_t n,
+                                                         double* __restrict__ out) {
+  if (!(comps[0].centered && comps[1].centered && comps[2].centered && comps[3].centered)) {
+    eval_hessian(comps, 4, x, n, out);
+    return;
+  }
+  const MWParams p = mw_of_table(comps);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double H[6];
     mw_hessian(p, x(i, 0), x(i, 1), x(i, 2), H);
@@ -243,20 +271,6 @@ __global__ void __launch_bounds__(128) k_eval_hessian_mw(MWParams p, Points x, i
     out[6 * n + i] = H[2];
     out[7 * n + i] = H[4];
     out[8 * n + i] = H[5];
-  }
-}
-
-__global__ void k_eval_hessian(const DevComp* comps, const DevLinear* lin, double t, int ncomp, Points x, int64_t n,
-                               double* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  DevComp* s = reinterpret_cast<DevComp*>(smem_raw);
-  stage_at_time(comps, lin, ncomp, t, s);
-  __syncthreads();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int c = 0; c < ncomp; ++c) comp_hessian(s[c], x(i, 0), x(i, 1), x(i, 2), H);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) out[k * n + i] = H[k];
   }
 }
 
@@ -590,7 +604,7 @@ gal_status gal_eval_points(const gal_potential* p, int32_t what, const double* x
       break;
     case GAL_EVAL_HESSIAN:
       if (p->is_mw) {
-        k_eval_hessian_mw<<<grid, block, 0, s>>>(p->mw, pts, n, out);
+        k_eval_hessian_mw<<<grid, block, 0, s>>>(p->d_comps, pts, n, out);
       } else {
         room((const void*)k_eval_hessian);
         k_eval_hessian<<<grid, block, smem, s>>>(p->d_comps, p->d_lin, t, p->n, pts, n, out);

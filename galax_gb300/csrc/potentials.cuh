@@ -518,6 +518,11 @@ struct MWParams {
   double Gm_n, rs_n;        // nucleus
 };
 
+// The same from a table of the four components (folded with the same operations).
+__device__ __forceinline__ MWParams mw_of_table(const DevComp* c) {
+  return MWParams{c[0].Gm, c[0].l1, c[0].l2sq, c[1].Gm, c[1].l1, c[1].inv_l1, c[2].Gm, c[2].l1, c[3].Gm, c[3].l1};
+}
+
 // The Milky Way gradient in four pieces, shared by MWPot::grad and the
 // four-warp team kernel (which evaluates the pieces on different warps), so
 // that both produce bitwise-identical results.

@@ -73,3 +73,33 @@ def test_orbits_among_many_spheres(method, others):
         torch.cuda.synchronize()
         assert torch.equal(out, run(from_component_array(arr, G=pot.G)))
         assert not torch.equal(out, first)
+
+
+@pytest.mark.parametrize("what", ["potential", "hessian"])
+@pytest.mark.parametrize("moved", [False, True])
+def test_milky_way_evaluation(what, moved):
+    import torch
+
+    import galax_gb300 as gx
+    from galax_gb300.potential import from_component_array
+
+    rng = np.random.default_rng(4)
+    pot = gx.MilkyWayPotential()
+    x = torch.as_tensor(rng.normal(size=(1000, 3)) * 9.0, device="cuda")
+    first = getattr(pot, what)(x).clone()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = getattr(pot, what)(x)
+    arr = _changed(pot, rng, 0.0)
+    if moved:
+        arr["origin"][1] = [0.5, 0.0, -0.25]
+    _update(pot, arr)
+    g.replay()
+    torch.cuda.synchronize()
+    want = getattr(from_component_array(arr, G=pot.G), what)(x)
+    if moved:  # the general code, compiled into another kernel: a few dozen roundings of 2^-53 at most
+        assert torch.all((out - want).abs() <= 1e-13 * want.reshape(1000, -1).norm(dim=1).reshape(-1, *[1] * (out.dim() - 1)))
+    else:
+        assert torch.equal(out, want)
+    assert not torch.equal(out, first)
