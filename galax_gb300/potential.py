@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import struct
 from collections.abc import Mapping
 from dataclasses import dataclass
 from typing import Any
@@ -31,6 +32,9 @@ from . import _lib
 
 G_GALACTIC = 4.498502151469553e-12  # kpc^3 / (Msun Myr^2): astropy's CODATA-2018 G in galactic units
 KMS_TO_KPC_MYR = 0.001022712165045695
+
+
+_KEY_G, _KEY_REC = struct.Struct("=d").pack, struct.Struct("=i6d").pack
 
 
 def _torch():
@@ -114,17 +118,22 @@ class AbstractPotential:
     def G(self) -> float:
         return self.constants["G"]
 
+    def _table_key(self) -> bytes:
+        """The component table's values, as bytes: a parameter may be an array that its owner changes in place."""
+        recs, slopes = self.components(), self.slopes()
+        key = _KEY_G(self.G) + b"".join([_KEY_REC(k, m, l1, l2, *o) for (k, m, l1, l2, o) in recs])
+        return key if slopes is None else key + slopes.tobytes()
+
     def handle(self) -> int:
         """The device-side ``gal_potential`` for the current CUDA device."""
         torch = _torch()
-        recs, slopes = self.components(), self.slopes()
-        key = (recs, self.G, None if slopes is None else slopes.tobytes())
+        key = self._table_key()
         if self._handle is not None and self._handle_key == key and self._handle_device == torch.cuda.current_device():
             return self._handle
         if not torch.cuda.is_available():
             raise _lib.GalaxGB300Error("no CUDA device: the galax_gb300 path has no CPU fallback")
         dev = torch.cuda.current_device()
-        arr = self.component_array()
+        arr, slopes = self.component_array(), self.slopes()
         self._release()
         L = _lib.load()
         h = C.c_void_p()
