@@ -172,7 +172,8 @@ class AbstractPotential:
         xt = torch.as_tensor(np.asarray(x, dtype=np.float64) if is_np else x)
         if xt.shape[-1] != 3:
             raise ValueError(f"positions must have a last axis of size 3, got shape {tuple(xt.shape)}")
-        return xt.reshape(-1, 3).to(device="cuda", dtype=torch.float64), xt.shape[:-1], is_np
+        pts = xt.reshape(-1, 3).to(device="cuda", dtype=torch.float64)
+        return pts.resolve_neg(), xt.shape[:-1], is_np  # values as they lie in memory: no lazily negated view
 
     @staticmethod
     def _out(t, is_np):

@@ -44,3 +44,17 @@ def test_milky_way_hessian_over_the_radii():
     # where it is below 1e-3 of the nucleus
     assert np.max(np.abs(H - ref) / scale) < 30 * 20 * 2.0**-53
     assert np.array_equal(H, np.swapaxes(H, 1, 2))
+
+
+def test_lazily_negated_view():
+    """The imaginary part of a conjugate is a view whose memory holds the negated values."""
+    import torch
+
+    import galax_gb300 as gx
+
+    z = torch.complex(*torch.randn((2, 300, 3), device="cuda", dtype=torch.float64))
+    x = z.conj().imag
+    assert x.is_neg()
+    mw = gx.MilkyWayPotential()
+    for what in ("potential", "gradient", "hessian"):
+        assert torch.equal(getattr(mw, what)(x), getattr(mw, what)(x.resolve_neg().contiguous()))
