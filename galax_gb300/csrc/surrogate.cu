@@ -249,8 +249,9 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   if (time_dependent(pot)) return fail(GAL_ERR_UNSUPPORTED, "time-dependent parameters: evaluation, integration and the orbit adjoint only");
   if (!std::isfinite(t0) || !std::isfinite(t1)) return fail(GAL_ERR_INVALID_ARGUMENT, "t0 and t1 must be finite");
   if (n == 0 || t0 == t1) return GAL_OK;
-  size_t need = 0;
-  gal_surrogate_workspace_size(n, &need);
+  size_t with_terms = 0;
+  gal_surrogate_workspace_size(n, &with_terms);
+  const size_t need = with_terms - align256(sizeof(double) * 3 * (size_t)n);  // slopes and positions alone
   if (!workspace || workspace_bytes < need) return fail(GAL_ERR_WORKSPACE, "workspace too small");
   double* F = static_cast<double*>(workspace);
   double* Yq = reinterpret_cast<double*>(static_cast<char*>(workspace) + align256(sizeof(double) * 7 * 6 * (size_t)n));
@@ -258,7 +259,8 @@ gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp,
   cudaStream_t caller = (cudaStream_t)stream;
   Side side;
   const SplitDev* spd = gal_split_device(near);
-  const bool apart = mlp && !spd;  // network and analytic term side by side
+  // network and analytic term side by side, if there is room to keep them apart; the results are the same bits
+  const bool apart = mlp && !spd && workspace_bytes >= with_terms;
   if (apart) {
     const cudaError_t es = side.create();
     if (es != cudaSuccess) return cuda_fail(es, "setting up the side stream");

@@ -500,8 +500,10 @@ GAL_API gal_status gal_split_eval(const gal_split* split, const double* x, int64
  * cores; NULL = none). Dopri5 with the constant step dt from t0 to t1 (the
  * last step clipped onto t1, as gal_integrate), advancing y[6][n] in place to
  * the final state. use_graph = 1 replays one captured CUDA graph per step.
- * Scratch from gal_surrogate_workspace_size (seven stage slopes and the stage
- * positions). */
+ * Scratch from gal_surrogate_workspace_size: seven stage slopes, the stage
+ * positions and the analytic accelerations (42 + 3 + 3 doubles per orbit, each
+ * part rounded up to 256 bytes). Without room for the last part the analytic and
+ * the network's term are evaluated one after the other, with the same results. */
 GAL_API gal_status gal_surrogate_workspace_size(int64_t n, size_t* bytes);
 GAL_API gal_status gal_integrate_surrogate(const gal_potential* pot, const gal_mlp* mlp, const gal_split* near,
                                            double dt, double t0, double t1, double* y, int64_t n, int32_t use_graph,

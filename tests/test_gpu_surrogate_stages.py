@@ -35,3 +35,38 @@ def test_zero_network_adds_nothing(n, with_near, host):
     direct = S.integrate(pot, mlp, y0, 0.0, 10.0, 1.0, near=near, use_graph=False)
     assert torch.equal(got, direct)
     assert torch.equal(got, plain)
+
+
+@pytest.mark.parametrize("use_graph", [0, 1])
+def test_workspace_without_the_terms_apart(use_graph):
+    """Seven slopes and the positions are enough; the analytic term then has no place
+    of its own and is evaluated before the network's, with the same bits."""
+    import ctypes as C
+
+    import torch
+
+    import galax_gb300 as gx
+    from galax_gb300 import _lib
+    from galax_gb300 import surrogate as S
+
+    n = 300
+    rng = np.random.default_rng(6)
+    pot, mlp = gx.MilkyWayPotential(), S.MLPSurrogate(S.init_params(3), 50.0, 2e-4)
+    y0 = torch.as_tensor(np.concatenate([rng.normal(size=(3, n)) * 8.0, rng.normal(size=(3, n)) * 0.12]), device="cuda")
+    L = _lib.load()
+    full = C.c_size_t()
+    _lib.check(L.gal_surrogate_workspace_size(n, C.byref(full)), "gal_surrogate_workspace_size")
+
+    def pad(b):
+        return (b + 255) // 256 * 256
+
+    least = pad(42 * 8 * n) + pad(3 * 8 * n)
+    out = []
+    for size in (full.value, least, least - 1):
+        y, ws = y0.clone(), torch.empty(size, dtype=torch.uint8, device="cuda")
+        out.append((L.gal_integrate_surrogate(pot.handle(), mlp.handle(), None, 1.0, 0.0, 10.0, y.data_ptr(), n, use_graph,
+                                              ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream), y))
+        torch.cuda.synchronize()
+    assert out[0][0] == out[1][0] == 0 and out[2][0] != 0
+    assert torch.equal(out[0][1], out[1][1]) and not torch.equal(out[0][1], y0)
+    assert torch.equal(out[2][1], y0)
