@@ -31,7 +31,8 @@ UNBOUNDED_MAX_STEPS = 2**20
 
 
 # Dopri8's scratch for saves (8 bytes each): kept with the workspace up to the first
-# bound (64 MB), allocated per call up to the second (4 GB), not used beyond.
+# bound (64 MB), allocated per call up to the second (4 GB; a workspace that the
+# caller gave grows to it instead), not used beyond or where memory does not do.
 SAVE_SCRATCH_KEPT = 2**23
 SAVE_SCRATCH_MAX = 2**29
 
@@ -323,15 +324,19 @@ def integrate(
     L = _lib.load()
     nbytes = C.c_size_t()
     total = shape[1] if save_offsets is not None else shape[1] * n
-    # a large save scratch (Dopri8, 8 bytes per save) is this call's alone instead of staying with the workspace
-    own = total > SAVE_SCRATCH_KEPT
-    if total > SAVE_SCRATCH_MAX:
-        total = 0
-    _lib.check(L.gal_integrate_workspace_size_saves(C.byref(cfg), n, total, C.byref(nbytes)),
-               "gal_integrate_workspace_size_saves")
-    if own and cfg.method == 8:
-        ws = torch.empty(nbytes.value, dtype=torch.uint8, device="cuda")
-    else:
+    ws = None
+    if cfg.method == 8 and 0 < total <= SAVE_SCRATCH_MAX:
+        _lib.check(L.gal_integrate_workspace_size_saves(C.byref(cfg), n, total, C.byref(nbytes)),
+                   "gal_integrate_workspace_size_saves")
+        try:
+            if total <= SAVE_SCRATCH_KEPT or workspace is not None:
+                ws = (workspace or _WS).get(nbytes.value)
+            else:  # this call's alone instead of staying with the kept workspace
+                ws = torch.empty(nbytes.value, dtype=torch.uint8, device="cuda")
+        except torch.cuda.OutOfMemoryError:  # saves inside the integration need no scratch
+            ws = None
+    if ws is None:
+        _lib.check(L.gal_integrate_workspace_size(C.byref(cfg), n, C.byref(nbytes)), "gal_integrate_workspace_size")
         ws = (workspace or _WS).get(nbytes.value)
     st = torch.cuda.current_stream().cuda_stream
     _lib.check(

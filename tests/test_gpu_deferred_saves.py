@@ -56,3 +56,59 @@ def test_same_bits_as_inline_saves(monkeypatch, pot_name, adaptive, n, n_saves, 
     for a, b in zip(deferred, inline):
         assert torch.equal(torch.nan_to_num(a.double(), nan=-7.0), torch.nan_to_num(b.double(), nan=-7.0))
     assert bool(torch.isfinite(deferred[0]).any())
+
+
+def _saves_case():
+    import galax_gb300 as gx
+
+    rng = np.random.default_rng(7)
+    y0 = np.concatenate([rng.normal(size=(40, 3)) * 8.0, rng.normal(size=(40, 3)) * 0.12], axis=1)
+    return gx.MilkyWayPotential(), y0, np.linspace(0.0, 200.0, 50), gx.Integrator().config()
+
+
+def test_no_memory_for_the_save_scratch(monkeypatch):
+    """A workspace that cannot grow to the scratch: saves inside the integration, same results."""
+    import torch
+
+    from galax_gb300 import dynamics as D
+
+    pot, y0, ts, cfg = _saves_case()
+    want = D.integrate(pot, y0, 0.0, 200.0, ts, cfg, workspace=D.Workspace())
+
+    class Small(D.Workspace):
+        def get(self, nbytes):
+            if nbytes > 40 * 50 * 8:
+                raise torch.cuda.OutOfMemoryError("no room")
+            sizes.append(nbytes)
+            return super().get(nbytes)
+
+    sizes = []
+    got = D.integrate(pot, y0, 0.0, 200.0, ts, cfg, workspace=Small())
+    monkeypatch.setattr(D, "_WS", Small())
+    kept = D.integrate(pot, y0, 0.0, 200.0, ts, cfg)
+    assert len(sizes) == 2
+    for res in (got, kept):
+        for a, b in zip(want, res):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("bound", ["SAVE_SCRATCH_KEPT", "SAVE_SCRATCH_MAX"])
+def test_the_callers_workspace_is_used(monkeypatch, bound):
+    import torch
+
+    from galax_gb300 import dynamics as D
+
+    pot, y0, ts, cfg = _saves_case()
+    want = D.integrate(pot, y0, 0.0, 200.0, ts, cfg, workspace=D.Workspace())
+    monkeypatch.setattr(D, bound, 100)
+
+    class Own(D.Workspace):
+        def get(self, nbytes):
+            sizes.append(nbytes)
+            return super().get(nbytes)
+
+    sizes = []
+    got = D.integrate(pot, y0, 0.0, 200.0, ts, cfg, workspace=Own())
+    assert len(sizes) == 1 and (sizes[0] > 40 * 50 * 8) == (bound == "SAVE_SCRATCH_KEPT")
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
