@@ -43,10 +43,17 @@ class AdjointResult:
 
 
 _WS = Workspace()
-# At most this much scratch for stored stages (12 GB); what a call needs beyond the
-# kept workspace's bound (256 MB) it allocates for itself.
+# At most this much scratch for stored stages (12 GB), and at most half of what is
+# free; what a call needs beyond the kept workspace's bound (256 MB) it allocates
+# for itself.
 STORED_STAGES_MAX = 12 << 30
 _KEPT_MAX = 256 << 20
+
+
+def _free_bytes() -> int:
+    """Device memory that torch could still hand out."""
+    torch = _torch()
+    return torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
 
 
 def _scratch(nbytes: int):
@@ -59,24 +66,30 @@ def _scratch(nbytes: int):
         return None
 
 
-def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None, stream=None):
+def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None, stream=None, stage_memory=None):
     torch = _torch()
     if stream is not None and stream != torch.cuda.current_stream().cuda_stream:
         with on_stream(stream):
-            return _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa, target_soa)
+            return _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa, target_soa, stage_memory=stage_memory)
     n = y0_soa.shape[1]
     cfg = _lib.solver_config(method, False, dt0=dt)
     L = _lib.load()
     h = pot.handle()
     nb = C.c_size_t()
-    _lib.check(L.gal_adjoint_workspace_size_stored(h, C.byref(cfg), float(t0), float(t1), int(k_ckpt), n,
-                                                   STORED_STAGES_MAX, C.byref(nb)),
-               "gal_adjoint_workspace_size_stored")
-    ws = _scratch(nb.value)
+
+    def size(extra: int) -> int:
+        _lib.check(L.gal_adjoint_workspace_size_stored(h, C.byref(cfg), float(t0), float(t1), int(k_ckpt), n,
+                                                       max(int(extra), 0), C.byref(nb)),
+                   "gal_adjoint_workspace_size_stored")
+        return nb.value
+
+    extra = STORED_STAGES_MAX if stage_memory is None else stage_memory
+    nbytes = size(extra)
+    if nbytes > _KEPT_MAX:
+        nbytes = size(min(extra, _free_bytes() // 2))
+    ws = _scratch(nbytes)
     if ws is None:  # no room for stored stages: checkpoints alone
-        _lib.check(L.gal_adjoint_workspace_size(h, C.byref(cfg), float(t0), float(t1), int(k_ckpt), n, C.byref(nb)),
-                   "gal_adjoint_workspace_size")
-        ws = _WS.get(nb.value)
+        ws = _WS.get(size(0))
     yT = torch.empty((6, n), dtype=torch.float64, device="cuda")
     gy = torch.empty((6, n), dtype=torch.float64, device="cuda")
     ncomp = len(pot.components())
@@ -95,12 +108,17 @@ def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None,
 
 
 def orbit_adjoint(pot: AbstractPotential, y0, t0: float, t1: float, *, dt: float, target=None, cotangent=None,
-                  method: int = 8, k_ckpt: int = 256) -> AdjointResult:
+                  method: int = 8, k_ckpt: int = 256, stage_memory: int | None = None) -> AdjointResult:
     """Forward + reverse sweep for n orbits with constant step ``dt``.
 
     Give ``target`` (n, 6) for the loss sum |y(t1) - target|^2, or ``cotangent``
     (n, 6) = dL/dy(t1) for any other loss. NumPy in, NumPy out; CUDA tensors stay
     on the device.
+
+    Scratch: checkpoints every ``k_ckpt`` steps and as many states between them,
+    48 bytes each per orbit. In the static Milky Way model the call also stores stages,
+    which makes it three times as fast, in up to ``stage_memory`` bytes (None:
+    12 GB or half of the free memory; 0: checkpoints alone).
     """
     torch = _torch()
     is_np = not isinstance(y0, torch.Tensor)
@@ -112,7 +130,7 @@ def orbit_adjoint(pot: AbstractPotential, y0, t0: float, t1: float, *, dt: float
         tgt = _as_cuda(target, torch.float64).reshape(-1, 6).t().contiguous()
     else:
         raise ValueError("give target or cotangent")
-    yT, gy, gp = _run(pot, y, t0, t1, dt, method, k_ckpt, lam, tgt)
+    yT, gy, gp = _run(pot, y, t0, t1, dt, method, k_ckpt, lam, tgt, stage_memory=stage_memory)
     loss = float(((yT - tgt) ** 2).sum()) if tgt is not None else None
     res = AdjointResult(yT.t(), gy.t(), gp, loss)
     if is_np:
@@ -127,7 +145,7 @@ class OrbitMap:
 
     @staticmethod
     def apply(pot: AbstractPotential, y0, params, t0: float, t1: float, dt: float, method: int = 8,
-              k_ckpt: int = 256):
+              k_ckpt: int = 256, stage_memory: int | None = None):
         torch = _torch()
 
         class _Fn(torch.autograd.Function):
@@ -149,7 +167,7 @@ class OrbitMap:
                 y0_, params_ = ctx.saved_tensors
                 y = y0_.detach().to(torch.float64).reshape(-1, 6).t().contiguous()
                 lam = gout.detach().to(torch.float64).reshape(-1, 6).t().contiguous()
-                _, gy, gp = _run(ctx.pot, y, t0, t1, dt, method, k_ckpt, lam_soa=lam)
+                _, gy, gp = _run(ctx.pot, y, t0, t1, dt, method, k_ckpt, lam_soa=lam, stage_memory=stage_memory)
                 return gy.t().reshape(y0_.shape), gp.reshape(params_.shape)
 
         return _Fn.apply(y0, params)

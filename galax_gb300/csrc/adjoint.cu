@@ -391,6 +391,17 @@ static size_t stored_step_bytes(int method, int64_t n) {
   return sizeof(double) * (size_t)((method == 8 ? Dopri8::S : Dopri5::S) * kStageDoubles) * (size_t)n;
 }
 
+// Steps whose stages `extra` bytes beyond L.total let a call store at a time, or 0:
+// checkpoints every k_ckpt steps where fewer than eight fit (unless they are all),
+// or where their segments' first states outnumber the checkpoint and segment areas.
+static int64_t stored_steps(const AdjLayout& L, int method, int64_t n, size_t extra) {
+  int64_t seg = (int64_t)(extra / stored_step_bytes(method, n));
+  if (seg > L.nsteps) seg = L.nsteps;
+  if (seg < 1 || (seg < 8 && seg != L.nsteps)) return 0;
+  const size_t states = (L.gp - L.ckpt) / (6 * sizeof(double) * (size_t)n);
+  return (size_t)((L.nsteps + seg - 1) / seg) <= states ? seg : 0;
+}
+
 }  // namespace gal
 
 using namespace gal;
@@ -417,10 +428,8 @@ gal_status gal_adjoint_workspace_size_stored(const gal_potential* pot, const gal
     if (st != GAL_OK || !pot->is_mw || n == 0) return st;
     std::vector<double> ts;
     time_grid(t0, t1, cfg->dt0, cfg->max_steps, ts);
-    const size_t per_step = stored_step_bytes(cfg->method, n);
-    size_t steps = max_extra / per_step;
-    if (steps > ts.size() - 1) steps = ts.size() - 1;
-    *bytes += steps * per_step;
+    const AdjLayout L = adj_layout(pot->n, 3, ts, k_ckpt, n);
+    *bytes += (size_t)stored_steps(L, cfg->method, n, max_extra) * stored_step_bytes(cfg->method, n);
     return GAL_OK;
   });
 }
@@ -465,14 +474,9 @@ gal_status gal_adjoint(const gal_potential* pot, const gal_solver_config* cfg, c
     a.k_ckpt = k_ckpt;
     a.n = n;
     a.lin = pot->d_lin;
-    // Stored stages when the workspace has room for at least eight steps of them
-    // (or all): below that, and for other tables, checkpoints every k_ckpt steps.
     if (pot->is_mw) {
-      int64_t seg = (int64_t)((workspace_bytes - L.total) / stored_step_bytes(cfg->method, n));
-      if (seg > L.nsteps) seg = L.nsteps;
-      const int64_t nseg = seg > 0 ? (L.nsteps + seg - 1) / seg : 0;
-      const size_t states = (L.gp - L.ckpt) / (6 * sizeof(double) * (size_t)n);  // the checkpoint and segment areas
-      if ((seg >= 8 || seg == L.nsteps) && (size_t)nseg <= states) {
+      const int64_t seg = stored_steps(L, cfg->method, n, workspace_bytes - L.total);
+      if (seg > 0) {
         StoredArgs b{};
         b.y0 = y0;
         b.lambda = lambda;

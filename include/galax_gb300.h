@@ -295,7 +295,9 @@ GAL_API gal_status gal_set_table_lanes(int32_t lanes);
 GAL_API gal_status gal_adjoint_workspace_size(const gal_potential* pot, const gal_solver_config* cfg, double t0, double t1,
                                       int32_t k_ckpt, int64_t n, size_t* bytes);
 /* The same, plus room for the stages of as many steps as max_extra bytes hold
- * (static Milky Way only: 1,040 bytes per orbit and Dopri8 step, 560 for Dopri5).
+ * (static Milky Way only: 1,040 bytes per orbit and Dopri8 step, 560 for Dopri5),
+ * or nothing more where gal_adjoint would not use them: fewer than eight steps, or
+ * more segments of such steps than the checkpoints' area has states for.
  * With such a workspace gal_adjoint stores the forward pass's stages instead of
  * evaluating them again in the reverse sweep; the gradients agree to rounding. */
 GAL_API gal_status gal_adjoint_workspace_size_stored(const gal_potential* pot, const gal_solver_config* cfg, double t0,

@@ -40,3 +40,55 @@ def test_matches_checkpointed_adjoint(method, n, seg, t1, given, monkeypatch):
     # sums of either sign over orbits and stages: relative to their largest per-row entry
     assert np.max(np.abs(stored.grad_params - plain.grad_params)[nz] / scale[nz]) < 1e-8
     assert np.array_equal(stored.grad_params[~nz], plain.grad_params[~nz])
+
+
+@pytest.mark.parametrize("method,per", [(5, 560), (8, 1040)])
+def test_no_scratch_that_would_not_be_used(method, per):
+    import ctypes as C
+
+    import galax_gb300 as gx
+    from galax_gb300 import _lib
+
+    L, h = _lib.load(), gx.MilkyWayPotential().handle()
+    cfg = _lib.solver_config(method, False, dt0=1.0)
+
+    def extra(n, steps, k_ckpt, most):
+        b, w = C.c_size_t(), C.c_size_t()
+        _lib.check(L.gal_adjoint_workspace_size(h, C.byref(cfg), 0.0, float(steps), k_ckpt, n, C.byref(b)), "size")
+        _lib.check(L.gal_adjoint_workspace_size_stored(h, C.byref(cfg), 0.0, float(steps), k_ckpt, n, most, C.byref(w)),
+                   "size_stored")
+        return w.value - b.value
+
+    n = 1_000_000
+    assert extra(n, 500, 256, 12 * n * per) == 12 * n * per
+    assert extra(n, 500, 256, 8 * n * per) == 8 * n * per
+    assert extra(n, 500, 256, 8 * n * per - 1) == 0           # seven steps: not worth it
+    assert extra(n, 5, 256, 8 * n * per - 1) == 5 * n * per   # all there are
+    assert extra(n, 5, 256, 5 * n * per - 1) == 0
+    # 50 segments of eight steps, but 21 + 20 states in the checkpoints' area
+    assert extra(n, 400, 20, 8 * n * per) == 0
+    assert extra(n, 400, 20, 10 * n * per) == 10 * n * per
+
+
+@pytest.mark.parametrize("free,stage_memory,stored", [(None, None, True), (None, 0, False), (10, None, False),
+                                                      (None, 9 * 300 * 1040, True), (None, 7 * 300 * 1040, False)])
+def test_memory_bounds(monkeypatch, free, stage_memory, stored):
+    import galax_gb300 as gx
+    from galax_gb300 import adjoint as A
+
+    sizes = []
+    scratch = A._scratch
+
+    def record(nbytes):
+        sizes.append(nbytes)
+        return scratch(nbytes)
+
+    monkeypatch.setattr(A, "_scratch", record)
+    monkeypatch.setattr(A, "_KEPT_MAX", 0)
+    if free is not None:
+        monkeypatch.setattr(A, "_free_bytes", lambda: free)
+    rng = np.random.default_rng(1)
+    y0 = np.concatenate([rng.normal(size=(300, 3)) * 8.0, rng.normal(size=(300, 3)) * 0.12], axis=1)
+    A.orbit_adjoint(gx.MilkyWayPotential(), y0, 0.0, 30.0, dt=1.0, cotangent=np.ones((300, 6)), k_ckpt=8,
+                    stage_memory=stage_memory)
+    assert (sizes[0] > 8 * 300 * 1040) == stored
