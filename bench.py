@@ -473,8 +473,7 @@ def run_uneven_dopri8(steps: int = 2, warmup: int = 1) -> dict:
             _, st, acc = step()
         ms = _timed(step, steps if blocks else 1, stream)
         res[blocks] = (ms, int(acc.sum()), int((st != 0).sum()))
-    # a fixed count: the automatic one, the library's default, cannot be set again
-    _lib.check(L.gal_set_team(32), "gal_set_team")
+    _lib.check(L.gal_set_team(-1), "gal_set_team")  # the library's defaults again
     _lib.check(L.gal_set_split_fraction(0.1), "gal_set_split_fraction")
     ms, accepted, bad = res[team]
     peak = fp64_peak()

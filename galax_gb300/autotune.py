@@ -54,6 +54,15 @@ def set_team(blocks: int) -> None:
     _lib.check(L.gal_set_team(int(blocks)), "gal_set_team")
 
 
+# The library's default: the number is chosen for each batch on the device.
+AUTOMATIC_TEAMS = -1
+
+
+def set_automatic_teams() -> None:
+    L = _lib.load()
+    _lib.check(L.gal_set_team(AUTOMATIC_TEAMS), "gal_set_team")
+
+
 # Fraction of every orbit's span covered by the first pass of the two-pass
 # schedule (gal_set_split_fraction; the library's default is 0.1). The first
 # pass's progress is what orders the second pass longest first: too short a
@@ -89,8 +98,12 @@ def tune(run: Callable[[], object], method: int, adaptive: bool,
     """Run ``run()`` under each launch-shape candidate ``repeats`` times and keep
     the one whose slowest run is fastest (no candidates: the shape is left as
     it is); then, for adaptive batches, the same over the number of SMs given to
-    four-warp teams (``teams``, by default the method's candidates) and, with the
-    best of those, over the first pass's split fraction. Returns the timings."""
+    four-warp teams (``teams``, by default the method's candidates, and the
+    library's own choice for each batch, ``team_blocks`` -1) and, with the best of
+    those, over the first pass's split fraction. Returns the timings. The settings
+    are the process's, for every later batch; ``set_automatic_teams`` gives the
+    choice back to the library. Batches of at most 64 orbits per SM run on teams
+    alone and depend on none of them."""
     timings = {}
     for cand in candidates:
         set_launch(method, adaptive, *cand)
@@ -108,9 +121,15 @@ def tune(run: Callable[[], object], method: int, adaptive: bool,
         for blocks in teams:
             set_team(blocks)
             tt[blocks] = _worst_ms(run, repeats)
+        set_automatic_teams()
+        automatic = _worst_ms(run, repeats)
         tbest = min(tt, key=tt.get)
-        set_team(tbest)
+        if automatic < tt[tbest]:
+            tbest = AUTOMATIC_TEAMS
+        else:
+            set_team(tbest)
         out["best"]["team_blocks"] = tbest
+        out["team_automatic_ms"] = round(automatic, 3)
         out["team_ms"] = {str(k): round(v, 3) for k, v in tt.items()}
         if splits:
             sp = {}

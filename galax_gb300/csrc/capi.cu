@@ -657,7 +657,7 @@ gal_status gal_integrate_workspace_size_saves(const gal_solver_config* cfg, int6
 }
 
 gal_status gal_set_team(int32_t blocks) {
-  if (blocks < 0 || blocks > 1024) return fail(GAL_ERR_INVALID_ARGUMENT, "team blocks must be in [0, 1024]");
+  if (blocks < -1 || blocks > 1024) return fail(GAL_ERR_INVALID_ARGUMENT, "team blocks must be in [-1, 1024]");
   g_team_blocks.store(blocks, std::memory_order_relaxed);
   return GAL_OK;
 }

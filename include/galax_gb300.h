@@ -264,15 +264,17 @@ GAL_API gal_status gal_dense_evaluate(const gal_potential* pot, int32_t method, 
  * threads at maximum occupancy (variant 0 for Dopri5, 2 for Dopri8). */
 GAL_API gal_status gal_set_launch(int32_t method, int32_t adaptive, int32_t block_threads, int32_t blocks_per_sm,
                                   int32_t variant);
-/* Four-warp team blocks (16 orbits each, two Runge-Kutta stages per round) in
- * the Milky Way model. blocks > 0 (at most the SM count - 1): small batches run
- * on teams alone, and the second pass of a larger two-pass batch gives `blocks`
- * SMs to teams, which take the longest orbits first, while the other SMs run one
- * thread per orbit; until it is set, that number is chosen for each batch on the
- * device from the first pass's step counts. 0 keeps every orbit on the one-thread
- * kernel with the launch shape of gal_set_launch. Results are bitwise identical
- * either way; the teams cut the serial latency of few or long orbits.
- * Process-wide. */
+/* Four-warp team blocks (16 orbits each, two Runge-Kutta stages per round), in the
+ * Milky Way model and for component tables of up to 16 components.
+ *   -1 (default): batches of at most 64 orbits per SM run on teams alone, in one
+ *      pass whatever cfg->schedule; the second pass of a larger two-pass Milky Way
+ *      batch gives some SMs to teams, which take the longest orbits first, while the
+ *      other SMs run one thread per orbit. How many is chosen for each batch on the
+ *      device from the first pass's step counts.
+ *   1..1024: the same with that many SMs (at most the SM count - 1) in the second pass.
+ *   0: every orbit on the one-thread kernel with the launch shape of gal_set_launch.
+ * Results are bitwise identical in each case; the teams cut the serial latency of
+ * few or long orbits. Process-wide. */
 GAL_API gal_status gal_set_team(int32_t blocks);
 /* Fraction of every orbit's span that the first pass of the two-pass schedule
  * (cfg->schedule = 1) covers before the orbits are ordered by their remaining

@@ -28,3 +28,16 @@ def goldens():
 
     with open(os.path.join(ROOT, "tests", "golden", "reference_goldens.json")) as f:
         return json.load(f)
+
+
+@pytest.fixture(autouse=True)
+def _library_defaults(request):
+    """Tests that set the process-wide scheduling leave the library's defaults behind."""
+    yield
+    if request.node.get_closest_marker("gpu"):
+        from galax_gb300 import _lib
+
+        L = _lib.load()
+        _lib.check(L.gal_set_team(-1), "gal_set_team")
+        _lib.check(L.gal_set_split_fraction(0.1), "gal_set_split_fraction")
+        _lib.check(L.gal_set_table_lanes(0), "gal_set_table_lanes")
