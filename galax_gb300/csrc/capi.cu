@@ -306,11 +306,15 @@ constexpr int kBuckets = 120;  // sixths of an octave of remaining step attempts
 // The first pass ends an orbit's part after this many step attempts at the
 // latest: the longest orbits' rates are known by then, and a tenth of their spans
 // would be thousands of steps, in which most lanes have nothing left to do
-// (65,536 uneven orbits, s: 0.59 at 512, 0.59-0.70 at 256, 0.60 at 1024, 0.65
-// without this bound).
+// (uneven orbits, s. Dopri5, 65,536 of them: 0.59 at 512, 0.59-0.70 at 256, 0.60 at
+// 1024, 0.65 without this bound. Dopri8 at 256 / 512 / 1024 / without: 16,384 of
+// them 0.41 / 0.42 / 0.44 / 0.48, 65,536 0.60 / 0.58 / 0.61 / 0.64, 262,144 1.35 /
+// 1.22 / 1.22 / 1.30).
 constexpr int kParkSteps = 512;
-// Lone-thread to team time per step attempt.
-constexpr float kTeamRatio5 = 2.7f, kTeamRatio8 = 3.5f;
+// Lone-thread to team time per step attempt. Dopri8, two batches of 65,536 uneven
+// orbits, s: 0.76 and 0.83 with 2.5, 0.62 and 0.67 with 3.0, 0.59 and 0.58 with 3.5,
+// 0.56 and 0.56 with 4.0 and 4.5; 262,144 of them 1.36 with 2.5 and 3.0, 1.22 above.
+constexpr float kTeamRatio5 = 2.7f, kTeamRatio8 = 4.0f;
 
 __global__ void k_sched_keys(const OrbitResume* __restrict__ r, int64_t n, unsigned* __restrict__ hist,
                              int* __restrict__ bucket) {
@@ -774,7 +778,12 @@ gal_status gal_integrate(const gal_potential* p, const gal_solver_config* cfg, c
   // Measured, constant step, 100 steps, ms on teams / one thread per orbit:
   // Dopri8 1.93 / 6.14 at 2,432 orbits, 2.50 / 6.12 at 4,864, 4.76 / 6.13 at
   // 9,728, 6.99 / 6.13 at 12,160; Dopri5 1.00 / 2.71, 1.26 / 2.71, 2.28 / 2.73,
-  // 3.28 / 2.73.
+  // 3.28 / 2.73. Tables at 4,864 and 9,728 orbits, teams' time of the single
+  // threads', constant (adaptive) Dopri8: power law with cutoff, disk and halo 0.47
+  // and 0.86 (0.48, 0.61), the power law alone 0.50 and 0.94 (0.68, 0.85), the six
+  // components of MilkyWayPotential2022 0.33 and 0.63 (0.30, 0.38), sixteen
+  // components 0.29 and 0.56 (0.26, 0.34); one component of any other kind 0.51-0.52
+  // and 0.98 (0.49, 0.51-0.75), which with Dopri5 is 0.54-0.58 and 1.00-1.02.
   if (team_blocks != 0 && n <= (int64_t)kTeamOrbitsPerSm * sms &&
       (p->is_mw || (p->n <= kTeamMaxComps && shape.table_lanes == 0))) {
     cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
