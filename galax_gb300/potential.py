@@ -20,6 +20,7 @@ callable parameters are rejected, as are unit systems other than "galactic".
 from __future__ import annotations
 
 import ctypes as C
+import marshal
 import math
 import struct
 from collections.abc import Mapping
@@ -37,10 +38,16 @@ KMS_TO_KPC_MYR = 0.001022712165045695
 _KEY_G, _KEY_REC = struct.Struct("=d").pack, struct.Struct("=i6d").pack
 
 
-def _torch():
-    import torch
+_torch_module = None
 
-    return torch
+
+def _torch():
+    global _torch_module
+    if _torch_module is None:
+        import torch
+
+        _torch_module = torch
+    return _torch_module
 
 
 @dataclass(frozen=True)
@@ -121,7 +128,10 @@ class AbstractPotential:
     def _table_key(self) -> bytes:
         """The component table's values, as bytes: a parameter may be an array that its owner changes in place."""
         recs, slopes = self.components(), self.slopes()
-        key = _KEY_G(self.G) + b"".join([_KEY_REC(k, m, l1, l2, *o) for (k, m, l1, l2, o) in recs])
+        try:
+            key = marshal.dumps((recs, self.G), 2)  # numbers and buffers by value; a third of packing's time
+        except ValueError:  # values of other types
+            key = _KEY_G(self.G) + b"".join([_KEY_REC(k, m, l1, l2, *o) for (k, m, l1, l2, o) in recs])
         return key if slopes is None else key + slopes.tobytes()
 
     def handle(self) -> int:
@@ -173,7 +183,9 @@ class AbstractPotential:
         if xt.shape[-1] != 3:
             raise ValueError(f"positions must have a last axis of size 3, got shape {tuple(xt.shape)}")
         pts = xt.reshape(-1, 3).to(device="cuda", dtype=torch.float64)
-        return pts.resolve_neg(), xt.shape[:-1], is_np  # values as they lie in memory: no lazily negated view
+        if pts.is_neg():  # a lazily negated view: its memory holds other values
+            pts = pts.resolve_neg()
+        return pts, xt.shape[:-1], is_np
 
     @staticmethod
     def _out(t, is_np):

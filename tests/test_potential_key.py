@@ -15,9 +15,10 @@ import galax_gb300 as gx
     lambda p: p.constants.__setitem__("G", 1.0),
 ])
 @pytest.mark.parametrize("composite", [False, True])
-def test_key_follows_values(change, composite):
+@pytest.mark.parametrize("step", [1, 2])  # an origin that is a strided view too
+def test_key_follows_values(change, composite, step):
     inner = gx.PlummerPotential(m_tot=1e9, r_s=1.0)
-    inner.m_tot, inner.origin = np.array(1e9), np.array([1.0, 2.0, 3.0])
+    inner.m_tot, inner.origin = np.array(1e9), np.array([1.0, 9.0, 2.0, 9.0, 3.0, 9.0])[:3 * step:step]
     pot = gx.CompositePotential([inner, gx.KeplerPotential(m_tot=1e8)]) if composite else inner
     before, again = pot._table_key(), pot._table_key()
     assert before == again
