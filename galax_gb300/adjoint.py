@@ -89,7 +89,8 @@ def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None,
         nbytes = size(min(extra, _free_bytes() // 2))
     ws = _scratch(nbytes)
     if ws is None:  # no room for stored stages: checkpoints alone
-        ws = _WS.get(size(0))
+        nbytes = size(0)
+        ws = _WS.get(nbytes)
     yT = torch.empty((6, n), dtype=torch.float64, device="cuda")
     gy = torch.empty((6, n), dtype=torch.float64, device="cuda")
     ncomp = len(pot.components())
@@ -100,7 +101,7 @@ def _run(pot, y0_soa, t0, t1, dt, method, k_ckpt, lam_soa=None, target_soa=None,
             h, C.byref(cfg), y0_soa.data_ptr(), float(t0), float(t1),
             lam_soa.data_ptr() if lam_soa is not None else None,
             target_soa.data_ptr() if target_soa is not None else None,
-            yT.data_ptr(), gy.data_ptr(), gp.data_ptr(), int(k_ckpt), n, ws.data_ptr(), ws.numel(), st,
+            yT.data_ptr(), gy.data_ptr(), gp.data_ptr(), int(k_ckpt), n, ws.data_ptr(), nbytes, st,
         ),
         "gal_adjoint",
     )

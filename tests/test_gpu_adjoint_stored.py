@@ -92,3 +92,25 @@ def test_memory_bounds(monkeypatch, free, stage_memory, stored):
     A.orbit_adjoint(gx.MilkyWayPotential(), y0, 0.0, 30.0, dt=1.0, cotangent=np.ones((300, 6)), k_ckpt=8,
                     stage_memory=stage_memory)
     assert (sizes[0] > 8 * 300 * 1040) == stored
+
+
+def test_a_larger_kept_workspace_changes_nothing(monkeypatch):
+    """stage_memory = 0 gives the checkpointed gradients also where an earlier call left room for stages."""
+    import galax_gb300 as gx
+    from galax_gb300 import adjoint as A
+
+    rng = np.random.default_rng(1)
+    y0 = np.concatenate([rng.normal(size=(30, 3)) * 8.0, rng.normal(size=(30, 3)) * 0.12], axis=1)
+
+    def run(stage_memory):
+        r = A.orbit_adjoint(gx.MilkyWayPotential(), y0, 0.0, 30.0, dt=1.0, cotangent=np.ones((30, 6)), k_ckpt=8,
+                            stage_memory=stage_memory)
+        return r.grad_y0, r.grad_params
+
+    monkeypatch.setattr(A, "_WS", A.Workspace())
+    fresh = run(0)
+    stored = run(None)
+    again = run(0)
+    for f, s, a in zip(fresh, stored, again):
+        np.testing.assert_array_equal(f, a)
+        assert not np.array_equal(f, s)
