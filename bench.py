@@ -707,11 +707,11 @@ def run_subhalos(args, n, rank, world, dist) -> dict | None:
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": {"workload": WORKLOADS["subhalos"].replace("1 Gyr", f"{t1:g} Myr"), "orbits_per_gpu": n,
                        "steps_per_orbit": nsteps, "orbits_not_finished": int((st != 0).sum())},
-            "roofline": {"bound": "fp64", "kernel": "k_integrate_table", "achieved": achieved,
+            "roofline": {"bound": "fp64", "kernel": "k_integrate_fixed", "achieved": achieved,
                          "peak": peak["tflops"], "unit": "TFLOP/s", "issue_ceiling": peak["issue_ceiling_tflops"],
                          "frac_of_issue_ceiling": achieved / peak["issue_ceiling_tflops"],
                          "frac": achieved / peak["tflops"], "flops_per_step": STEP_FLOPS_MW_SUBHALOS[5],
-                         "note": "nominal flops; the spheres are summed in 64-bit integers, so above 1 is possible"},
+                         "note": "nominal flops; most of a sphere's term is 64-bit integer work, so above 1 is possible"},
             "clocks": clk, "gpu_launches": args.steps}
 
 

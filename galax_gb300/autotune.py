@@ -43,9 +43,9 @@ def set_launch(method: int, adaptive: bool, block: int, per_sm: int, variant: in
 
 # SMs given to four-warp teams for the longest orbits (second pass of a
 # two-pass adaptive Milky Way batch, gal_set_team), per method. On the
-# 262,144-orbit headline batch (ms, Dopri5: 24 -> 1,175, 28 -> 1,100, 32 -> 1,102,
-# 40 -> 1,113; Dopri8: 6 -> 1,430, 8 -> 1,431, 10 -> 1,422, 12 -> 1,431,
-# 16 -> 1,429, none -> 1,887).
+# 262,144-orbit headline batch (ms, Dopri5: 24 -> 1,172, 28 -> 1,095, 32 -> 1,099,
+# 40 -> 1,106, the library's own choice 1,095; Dopri8: 6 -> 1,430, 8 -> 1,421,
+# 10 -> 1,420, 12 -> 1,430, 16 -> 1,432, its own choice 1,220, none -> 1,891).
 DEFAULT_TEAMS = {5: (24, 28, 32, 40), 8: (6, 8, 10, 12, 16)}
 
 

@@ -281,14 +281,21 @@ GAL_API gal_status gal_set_team(int32_t blocks);
  * work (default 0.1, allowed [0.001, 0.9]). Results are bitwise identical for
  * any value; it only moves work between the passes. Process-wide. */
 GAL_API gal_status gal_set_split_fraction(double fraction);
-/* Orbits per thread or warp for component tables (composites other than the
- * specialised Milky Way kernel) in gal_integrate: 1 runs one thread per orbit;
- * 32 runs one warp per orbit, its lanes splitting the components and reducing
- * the gradient with warp shuffles; 0 (default) takes a warp per orbit when the
- * table has at least 32 components and the batch is too small to give every
- * SM sub-partition a warp of 32 orbits (fewer than 128 orbits per SM).
- * The two differ only in the order of the component sum (rounding).
- * Process-wide. galax evaluates a composite by summing its components
+/* How gal_integrate evaluates component tables (composites other than the
+ * specialised Milky Way kernel).
+ *   0 (default): with constant steps and static parameters, a table's Plummer
+ *      spheres, if they are at least 32, through 64-bit integers on 1 to 32 lanes
+ *      per orbit (each sphere's term within 5 roundings of 2^-53; in FP64 it is
+ *      within about 10). Otherwise tables of up to 16 components on teams where
+ *      gal_set_team says so, tables of at least 32 components on a warp per orbit
+ *      while the batch is too small to give every SM sub-partition a warp of 32
+ *      orbits (fewer than 128 orbits per SM), and the rest on a thread per orbit.
+ *   1: one thread per orbit, every component in FP64.
+ *   32: one warp per orbit, its lanes splitting the components and reducing the
+ *      gradient with warp shuffles; the spheres as with 0.
+ * The results differ by rounding (of the spheres' terms, and of the order of the
+ * component sum); teams and a thread per orbit give the same bits. Process-wide.
+ * galax evaluates a composite by summing its components
  * (src/galax/potential/_src/base_multi.py:48-55). */
 GAL_API gal_status gal_set_table_lanes(int32_t lanes);
 
