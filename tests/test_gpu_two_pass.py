@@ -117,3 +117,49 @@ def test_automatic_teams_can_be_set_again():
     _set_team(8)
     autotune.set_automatic_teams()
     assert L.gal_set_team(-2) != 0 and L.gal_set_team(1025) != 0
+
+
+@pytest.mark.parametrize("method", [5, 8])
+def test_without_a_workspace(method):
+    """gal_integrate_noalloc with two passes, call after call on other orbits and
+    replayed from a graph: its array is reused by every call."""
+    import ctypes as C
+
+    import torch
+
+    import galax_gb300 as gx
+    from galax_gb300 import _lib
+    from galax_gb300.dynamics import Workspace, integrate
+
+    mw, L, cfg = gx.MilkyWayPotential(), _lib.load(), _cfg(method, True, "csr")
+    b = _batch("csr")
+    y0 = torch.as_tensor(b.y0, device="cuda").t().contiguous()
+    t0, t1 = torch.as_tensor(b.t0, device="cuda"), torch.as_tensor(b.t1, device="cuda").contiguous()
+    ts = torch.linspace(0.0, 50.0, 5, dtype=torch.float64, device="cuda")
+    out = torch.empty((6, 5, N), dtype=torch.float64, device="cuda")
+    status = torch.empty(N, dtype=torch.int32, device="cuda")
+    steps = torch.empty(N, dtype=torch.int64, device="cuda")
+
+    def call():
+        _lib.check(L.gal_integrate_noalloc(
+            mw.handle(), C.byref(cfg), y0.data_ptr(), t0.data_ptr(), t1.data_ptr(), None, ts.data_ptr(), 5,
+            out.data_ptr(), status.data_ptr(), steps.data_ptr(), None, N, torch.cuda.current_stream().cuda_stream),
+            "gal_integrate_noalloc")
+
+    def check():
+        torch.cuda.synchronize()
+        want = integrate(mw, y0, t0, t1, ts, cfg, soa=True, workspace=Workspace())
+        for a, w in zip((out, status, steps), want):
+            assert torch.equal(a, w)
+
+    for k in range(2):
+        y0.copy_(y0.roll(1777 * k, dims=1))
+        call()
+        check()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call()
+    for k in range(2):
+        y0.copy_(y0.roll(311, dims=1) * (1.0 - 0.01 * k))
+        g.replay()
+        check()
